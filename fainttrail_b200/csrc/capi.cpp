@@ -247,6 +247,24 @@ int ft_b200_stage_dev(ft_b200_ctx* ctx, const float* d_sub, int width, int heigh
     });
 }
 
+namespace {
+// The plan the device makes for a pass in a tile shape (0: the automatic
+// choice); a shape that does not take the pass falls back to the automatic
+// choice, as ft_b200_set_tile_shape does for the device.
+static ftb::StackPlan plan_on_host(int w, int h, int n, const int* dx, const int* dy, int m, int min_count, int shape) {
+    constexpr int kB200SmemOptin = 232448;  // 227 KB of shared memory per block
+    ftb::StackPlan plan;
+    if (ftb::make_streamed_pass(w, h, n, dx, dy, m, min_count, shape, false, plan)) return plan;
+    const std::vector<int> order = ftb::motion_order(dx, dy, m, n, 4.0, 4.0);
+    ftb::StackConfig cfg = ftb::choose_stack_config(n, dx, dy, order, kB200SmemOptin);
+    if (shape > 0 && shape != ftb::kStreamShape) {
+        const ftb::StackConfig asked = ftb::stack_shape_config(shape, kB200SmemOptin);
+        if (ftb::stack_shape_fits(asked, n)) cfg = asked;
+    }
+    return ftb::make_stack_plan(w, h, n, dx, dy, m, min_count, order, cfg);
+}
+}  // namespace
+
 int ft_b200_emulate_stack(const float* frames, int width, int height, int nframes, const int* dx, const int* dy,
                           int motions, int min_count, int shape, float* max_snr, int* best_v) {
     try {
@@ -260,15 +278,7 @@ int ft_b200_emulate_stack(const float* frames, int width, int height, int nframe
             std::fill(best_v, best_v + pixels, -1);
             return FT_B200_OK;
         }
-        constexpr int kB200SmemOptin = 232448;  // 227 KB of shared memory per block
-        // a fixed shape whose windows do not fit falls back to the automatic
-        // choice, as ft_b200_set_tile_shape does for the device
-        ftb::StackConfig cfg = ftb::choose_stack_config(width, height, nframes, kB200SmemOptin);
-        if (shape > 0 && ftb::stack_shape_fits(ftb::stack_shape_config(shape, kB200SmemOptin), nframes))
-            cfg = ftb::stack_shape_config(shape, kB200SmemOptin);
-        const ftb::StackPlan plan =
-            ftb::make_stack_plan(width, height, nframes, dx, dy, motions, min_count,
-                                 ftb::motion_order(dx, dy, motions, nframes, 4.0, 4.0), cfg);
+        const ftb::StackPlan plan = plan_on_host(width, height, nframes, dx, dy, motions, min_count, shape);
         ftb::emulate_stack_pass(plan, frames, max_snr, best_v);
         return FT_B200_OK;
     } catch (const std::exception& e) {
@@ -293,12 +303,16 @@ int ft_b200_plan_stats(int width, int height, int nframes, const int* dx, const 
         if (!dx || !dy || !stats || width < 1 || height < 1 || nframes < 1 || motions < 1)
             throw std::runtime_error("plan_stats: malformed pass");
         if (shape < 0 || shape > ftb::kStackShapes) throw std::runtime_error("plan_stats: unknown tile shape");
-        constexpr int kB200SmemOptin = 232448;
-        ftb::StackConfig cfg = ftb::choose_stack_config(width, height, nframes, kB200SmemOptin);
-        if (shape > 0 && ftb::stack_shape_fits(ftb::stack_shape_config(shape, kB200SmemOptin), nframes))
-            cfg = ftb::stack_shape_config(shape, kB200SmemOptin);
-        const ftb::StackPlan plan = ftb::make_stack_plan(width, height, nframes, dx, dy, motions, 1,
-                                                         ftb::motion_order(dx, dy, motions, nframes, 4.0, 4.0), cfg);
+        const ftb::StackPlan plan = plan_on_host(width, height, nframes, dx, dy, motions, 1, shape);
+        if (!plan.stream.empty()) {
+            const ftb::StreamPlan& q = plan.stream;
+            const long long slots = static_cast<long long>(q.slot_motion.size());
+            stats[0] = stats[1] = static_cast<long long>(q.groups.size());
+            stats[2] = stats[4] = slots;
+            stats[3] = std::count(q.slot_motion.begin(), q.slot_motion.end(), -1);
+            stats[5] = static_cast<long long>(ftb::stream_frames(nframes, q.rows)) * q.rows * ftb::kStreamPitch * 4;
+            return FT_B200_OK;
+        }
         long long fast = 0, pads = 0, fast_slots = 0;
         for (const auto& g : plan.groups) {
             fast += g.rows_fast;

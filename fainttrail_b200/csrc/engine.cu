@@ -226,20 +226,37 @@ enum Slot { kFrames = 0, kBest, kArg, kMax, kBestV, kStageOut, kSky, kMask, kDes
 
 namespace {
 
+size_t align256(size_t b) { return (b + 255) / 256 * 256; }
+
+// A buffer a call can do without: empty where the budget or the device has no
+// room for it.
+DevBuf spare_buffer(Context& c, size_t bytes, const char* what) {
+    if (c.used() + bytes > c.budget()) return DevBuf();
+    try {
+        return DevBuf(&c, bytes, what);
+    } catch (const std::exception&) {
+        return DevBuf();
+    }
+}
+
 // Launch a planned pass in group ranges; between ranges the progress callback
 // is asked (fraction of groups done), as the reference CUDA backend does between
-// its launches (backend_cuda.cu:167-173).
-void run_plan(Context& c, const StackPlan& plan, const float* d_frames, float* d_max, int* d_bv,
+// its launches (backend_cuda.cu:167-173). keys: a streamed pass's running maxima,
+// where it runs in parts.
+void run_plan(Context& c, const StackPlan& plan, const float* d_frames, float* d_max, int* d_bv, const DevBuf& keys,
               const Progress& progress) {
     StackPlanDev dev;
     dev.upload(plan, c.stream());
-    const int ng = static_cast<int>(plan.groups.size());
+    const bool streamed = !plan.stream.empty();
+    const int ng = plan.ngroups();
     const int chunks = progress ? std::min(ng, 16) : 1;
+    const size_t pixels = static_cast<size_t>(plan.w) * plan.h;
+    const int splits = streamed && keys ? stream_splits({&plan}, c.sms()) : 1;
     float* d_best = nullptr;
     int* d_arg = nullptr;
-    if (chunks > 1) {
-        d_best = c.scratch(kBest, sizeof(float) * static_cast<size_t>(plan.w) * plan.h, "stack maxima").as<float>();
-        d_arg = c.scratch(kArg, sizeof(int) * static_cast<size_t>(plan.w) * plan.h, "stack argmax").as<int>();
+    if (!streamed && chunks > 1) {
+        d_best = c.scratch(kBest, sizeof(float) * pixels, "stack maxima").as<float>();
+        d_arg = c.scratch(kArg, sizeof(int) * pixels, "stack argmax").as<int>();
     }
     try {
         const int span = c.span_begin("kernel");
@@ -258,9 +275,16 @@ void run_plan(Context& c, const StackPlan& plan, const float* d_frames, float* d
             bp.arg = d_arg;
             bp.max_snr = d_max;
             bp.best_v = d_bv;
-            DevBuf& desc = c.scratch(kDesc, batch_desc_bytes(1), "stack descriptors");
-            stack_launch_batch({bp}, desc.as<unsigned char>(), desc.bytes(), c.err_flag(), c.sms(), c.stream());
-            ++c.launches;
+            bp.keys = keys.as<unsigned long long>();
+            DevBuf& desc =
+                c.scratch(kDesc, streamed ? stream_desc_bytes(1) : batch_desc_bytes(1), "stack descriptors");
+            if (streamed) {
+                c.launches += stream_launch({bp}, splits, desc.as<unsigned char>(), desc.bytes(), c.err_flag(), c.sms(),
+                                            c.stream());
+            } else {
+                stack_launch_batch({bp}, desc.as<unsigned char>(), desc.bytes(), c.err_flag(), c.sms(), c.stream());
+                ++c.launches;
+            }
             if (progress) {
                 c.check_kernel_error("stack kernel");
                 if (!progress(static_cast<double>(q + 1) / chunks, "stack")) throw Cancelled();
@@ -290,14 +314,23 @@ void stack_pass_device(Context& c, const float* d_frames, int pitch, int w, int 
         return;
     }
     const double t0 = wall_seconds();
-    const StackConfig cfg = choose_stack_config(w, h, n, c.smem_optin());
-    const std::vector<int> order = motion_order(dx, dy, m, n, 4.0, 4.0);
     (void)vel;
     (void)tmax;
-    StackPlan plan = make_stack_plan(w, h, n, dx, dy, m, min_count, order, cfg);
+    StackPlan plan;
+    DevBuf keys;
+    bool streamed = make_streamed_pass(w, h, n, dx, dy, m, min_count, stack_shape(), false, plan);
+    if (streamed && (progress || stream_splits({&plan}, c.sms()) > 1)) {
+        keys = spare_buffer(c, sizeof(unsigned long long) * static_cast<size_t>(w) * h, "stack maxima");
+        streamed = keys || !progress;  // without room for them: one part, one work item a tile
+    }
+    if (!streamed) {
+        const std::vector<int> order = motion_order(dx, dy, m, n, 4.0, 4.0);
+        plan = make_stack_plan(w, h, n, dx, dy, m, min_count, order,
+                               choose_stack_config(n, dx, dy, order, c.smem_optin()));
+    }
     plan.pitch = pitch;
     c.host_time("setup", wall_seconds() - t0);
-    run_plan(c, plan, d_frames, d_max_snr, d_best_v, progress);
+    run_plan(c, plan, d_frames, d_max_snr, d_best_v, keys, progress);
 }
 
 void stack_pass_host(Context& c, const float* frames, int w, int h, int n, const int* dx, const int* dy, int m,
@@ -393,7 +426,7 @@ std::map<std::tuple<int, int, int, int>, int> g_tuned;  // (frames, motions, wid
 // more than a better shape can save.
 constexpr double kTuneMinAdds = 5e11;
 
-// The tile shape for a pass: the cached choice for its (frames, motions, size),
+// The tile shape for a pass that is not streamed: the cached choice for its (frames, motions, size),
 // else, for a large pass, every shape whose windows fit is planned and timed on a
 // band of tile rows in the middle of the image (about 8 tiles per SM, so each
 // probe is a few per cent of the pass), and the fastest per output pixel wins.
@@ -404,13 +437,14 @@ int autotune_shape(Context& c, const PassJob& j) {
     if (static_cast<double>(j.m) * j.n * j.w * j.h < kTuneMinAdds) return 0;
     const auto key = std::make_tuple(j.n, j.m, j.w, j.h);
     {
+        // kStreamShape there: another pass of this size was streamed
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tuned.find(key);
-        if (it != g_tuned.end()) return it->second;
+        if (it != g_tuned.end() && it->second != kStreamShape) return it->second;
     }
     std::vector<int> cands;
     for (int s = 1; s <= kStackShapes; ++s)
-        if (stack_shape_fits(stack_shape_config(s, c.smem_optin()), j.n)) cands.push_back(s);
+        if (s != kStreamShape && stack_shape_fits(stack_shape_config(s, c.smem_optin()), j.n)) cands.push_back(s);
     int best = cands.empty() ? 0 : cands[0];
     if (cands.size() > 1) {
         const double t0 = wall_seconds();
@@ -487,57 +521,66 @@ void clear_tuned_shapes() {
 
 namespace {
 
-// The configuration a pass takes when no probe has to run first: a fixed
-// shape, the autotuner's cached choice, or the frame-count rule for a pass too
-// small to tune. False when the autotuner still has to time the pass's kind.
-bool known_config(const Context& c, const PassJob& j, StackConfig& cfg) {
-    int shape = 0;
+// The shape a pass that is not streamed takes when no probe has to run first: the
+// autotuner's cached choice, or 0 (choose_stack_config) for a fixed shape or a
+// pass too small to tune. False when the autotuner still has to time the pass's
+// kind.
+bool known_shape(const PassJob& j, int& shape) {
+    shape = 0;
     if (stack_shape() == 0 && static_cast<double>(j.m) * j.n * j.w * j.h >= kTuneMinAdds) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tuned.find(std::make_tuple(j.n, j.m, j.w, j.h));
-        if (it == g_tuned.end()) return false;
+        if (it == g_tuned.end() || it->second == kStreamShape) return false;
         shape = it->second;
     }
-    cfg = shape > 0 ? stack_shape_config(shape, c.smem_optin()) : choose_stack_config(j.w, j.h, j.n, c.smem_optin());
     return true;
 }
 
-bool same_config(const StackConfig& a, const StackConfig& b) {
-    return a.ty == b.ty && a.p == b.p && a.tile_w == b.tile_w && a.wp == b.wp && a.merge == b.merge &&
-           a.rows == b.rows && a.smem_bytes == b.smem_bytes;
+StackPlan resident_plan(int smem_optin, const PassJob& j, int shape) {
+    const std::vector<int> order = motion_order(j.dx.data(), j.dy.data(), j.m, j.n, 4.0, 4.0);
+    return make_stack_plan(j.w, j.h, j.n, j.dx.data(), j.dy.data(), j.m, j.min_count, order,
+                           shape > 0 ? stack_shape_config(shape, smem_optin)
+                                     : choose_stack_config(j.n, j.dx.data(), j.dy.data(), order, smem_optin));
+}
+
+// The plan of a job: streamed where its motions pack for it, else by known_shape
+// (an empty plan, m = 0, where the autotuner has to run first).
+StackPlan plan_job(int smem_optin, const PassJob& j) {
+    StackPlan plan;
+    int shape = 0;
+    if (!make_streamed_pass(j.w, j.h, j.n, j.dx.data(), j.dy.data(), j.m, j.min_count, stack_shape(), true, plan)) {
+        if (!known_shape(j, shape)) return StackPlan();
+        plan = resident_plan(smem_optin, j, shape);
+    }
+    plan.pitch = j.pitch;
+    return plan;
 }
 
 }  // namespace
 
 PlanAhead plan_ahead(Context& c, std::vector<PassJob> tables) {
     PlanAhead out;
+    out.shape = stack_shape();
     out.plans.resize(tables.size());
     auto jobs = std::make_shared<std::vector<PassJob>>(std::move(tables));
-    auto cfgs = std::make_shared<std::vector<StackConfig>>(jobs->size());
     auto promises = std::make_shared<std::vector<std::promise<StackPlan>>>();
     std::vector<size_t> todo;
     for (size_t k = 0; k < jobs->size(); ++k)
-        if ((*jobs)[k].min_count <= (*jobs)[k].n && known_config(c, (*jobs)[k], (*cfgs)[k])) todo.push_back(k);
+        if ((*jobs)[k].min_count <= (*jobs)[k].n) todo.push_back(k);
     promises->resize(todo.size());
     for (size_t q = 0; q < todo.size(); ++q) out.plans[todo[q]] = (*promises)[q].get_future().share();
     const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
     const size_t workers = std::min<size_t>(hw, todo.size());
     for (size_t wkr = 0; wkr < workers; ++wkr)
-        std::thread([jobs, cfgs, promises, todo, wkr, workers] {
+        std::thread([jobs, promises, todo, wkr, workers, smem = c.smem_optin()] {
             for (size_t q = wkr; q < todo.size(); q += workers) {
-                const PassJob& j = (*jobs)[todo[q]];
                 try {
-                    StackPlan plan = make_stack_plan(j.w, j.h, j.n, j.dx.data(), j.dy.data(), j.m, j.min_count,
-                                                     motion_order(j.dx.data(), j.dy.data(), j.m, j.n, 4.0, 4.0),
-                                                     (*cfgs)[todo[q]]);
-                    plan.pitch = j.pitch;
-                    (*promises)[q].set_value(std::move(plan));
+                    (*promises)[q].set_value(plan_job(smem, (*jobs)[todo[q]]));
                 } catch (...) {
                     (*promises)[q].set_exception(std::current_exception());
                 }
             }
         }).detach();
-    out.cfgs = *cfgs;
     return out;
 }
 
@@ -557,65 +600,108 @@ void stack_passes_device(Context& c, std::vector<PassJob>& jobs, PlanAhead* ahea
         FTB_CHECK(cudaStreamSynchronize(c.stream()));
         return;
     }
-    // tile shapes first (probes run on the stream, before this batch's launches)
-    std::vector<int> shapes_for(jobs.size(), 0);
-    for (size_t k = 0; k < jobs.size(); ++k) shapes_for[k] = autotune_shape(c, jobs[k]);
     const double t0 = wall_seconds();
-    // plans on host threads (the GPU keeps running whatever was queued before)
+    // plans made ahead, or on host threads now (the GPU keeps running whatever
+    // was queued before)
     std::vector<StackPlan> plans(jobs.size());
+    const bool use = ahead && ahead->shape == stack_shape();
     const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
     const size_t workers = std::min<size_t>(hw, jobs.size());
     std::vector<std::thread> pool;
     std::vector<std::exception_ptr> errs(workers);
-    for (size_t wkr = 0; wkr < workers; ++wkr)
-        pool.emplace_back([&, wkr] {
-            try {
-                for (size_t k = wkr; k < jobs.size(); k += workers) {
-                    const PassJob& j = jobs[k];
-                    const StackConfig cfg = shapes_for[k] > 0 ? stack_shape_config(shapes_for[k], c.smem_optin())
-                                                              : choose_stack_config(j.w, j.h, j.n, c.smem_optin());
-                    // a plan made ahead for the same configuration (the tables are the job's)
-                    if (ahead && k < ahead->plans.size() && ahead->plans[k].valid() &&
-                        same_config(ahead->cfgs[k], cfg)) {
-                        plans[k] = ahead->plans[k].get();
-                        plans[k].pitch = j.pitch;
-                        continue;
-                    }
-                    plans[k] = make_stack_plan(j.w, j.h, j.n, j.dx.data(), j.dy.data(), j.m, j.min_count,
-                                               motion_order(j.dx.data(), j.dy.data(), j.m, j.n, 4.0, 4.0), cfg);
-                    plans[k].pitch = j.pitch;
+    auto work = [&](size_t wkr) {
+        try {
+            for (size_t k = wkr; k < jobs.size(); k += workers) {
+                if (use && k < ahead->plans.size() && ahead->plans[k].valid()) {
+                    plans[k] = ahead->plans[k].get();  // the tables are the job's
+                    plans[k].pitch = jobs[k].pitch;
+                } else {
+                    plans[k] = plan_job(c.smem_optin(), jobs[k]);
                 }
-            } catch (...) {
-                errs[wkr] = std::current_exception();
             }
-        });
-    for (auto& t : pool) t.join();
+        } catch (...) {
+            errs[wkr] = std::current_exception();
+        }
+    };
+    if (workers == 1) {
+        work(0);
+    } else {
+        for (size_t wkr = 0; wkr < workers; ++wkr) pool.emplace_back(work, wkr);
+        for (auto& t : pool) t.join();
+    }
     for (auto& e : errs)
         if (e) std::rethrow_exception(e);
     c.host_time("plans", wall_seconds() - t0);
+    // the passes left to the autotuner (its probes run on the stream, before
+    // this batch's launches); a streamed pass of that size is noted beside them
+    for (size_t k = 0; k < jobs.size(); ++k) {
+        const PassJob& j = jobs[k];
+        if (!plans[k].stream.empty()) {
+            if (stack_shape() == 0 && plans[k].adds >= kTuneMinAdds) {
+                std::lock_guard<std::mutex> lk(g_tune_mu);
+                g_tuned.emplace(std::make_tuple(j.n, j.m, j.w, j.h), kStreamShape);
+            }
+            continue;
+        }
+        if (plans[k].m > 0) continue;
+        plans[k] = resident_plan(c.smem_optin(), j, autotune_shape(c, j));
+        plans[k].pitch = j.pitch;
+    }
+    // the streamed passes, small ones cut into several work items a tile, whose
+    // maxima then merge in global keys (without room for those: one item a tile)
+    std::vector<size_t> streamed;
+    std::vector<const StackPlan*> stream_plans;
+    size_t key_bytes = 0;
+    for (size_t k = 0; k < jobs.size(); ++k) {
+        if (plans[k].stream.empty()) continue;
+        streamed.push_back(k);
+        stream_plans.push_back(&plans[k]);
+        key_bytes += align256(sizeof(unsigned long long) * static_cast<size_t>(jobs[k].w) * jobs[k].h);
+    }
+    int splits = streamed.empty() ? 1 : stream_splits(stream_plans, c.sms());
+    DevBuf keys;
+    if (splits > 1) {
+        keys = spare_buffer(c, key_bytes, "stack maxima");
+        if (!keys) splits = 1;
+    }
     std::vector<StackPlanDev> devs(jobs.size());
     try {
         for (size_t k = 0; k < jobs.size(); ++k) devs[k].upload(plans[k], c.stream());
-        // one persistent launch per kernel shape
+        auto pass = [&](size_t k) {
+            BatchPass bp;
+            bp.plan = &plans[k];
+            bp.dev = &devs[k];
+            bp.frames = jobs[k].d_frames;
+            bp.g0 = 0;
+            bp.g1 = plans[k].ngroups();
+            bp.max_snr = jobs[k].d_max;
+            bp.best_v = jobs[k].d_bv;
+            return bp;
+        };
+        const int span = c.span_begin("kernel");
+        std::vector<BatchPass> batch;
+        if (!streamed.empty()) {
+            unsigned char* at = keys.as<unsigned char>();
+            for (size_t k : streamed) {
+                batch.push_back(pass(k));
+                if (!keys) continue;
+                batch.back().keys = reinterpret_cast<unsigned long long*>(at);
+                at += align256(sizeof(unsigned long long) * static_cast<size_t>(jobs[k].w) * jobs[k].h);
+            }
+            DevBuf& desc = c.scratch(kDesc, stream_desc_bytes(static_cast<int>(batch.size())), "stack descriptors");
+            c.launches += stream_launch(batch, splits, desc.as<unsigned char>(), desc.bytes(), c.err_flag(), c.sms(),
+                                        c.stream());
+        }
+        // the others: one persistent launch per kernel shape
         auto key = [](const StackConfig& q) { return std::make_pair((q.ty * 1000 + q.p) * 2 + q.merge, q.tile_w); };
         std::vector<std::pair<int, int>> shapes;
         for (const auto& p : plans)
-            if (std::find(shapes.begin(), shapes.end(), key(p.cfg)) == shapes.end()) shapes.push_back(key(p.cfg));
-        const int span = c.span_begin("kernel");
+            if (p.stream.empty() && std::find(shapes.begin(), shapes.end(), key(p.cfg)) == shapes.end())
+                shapes.push_back(key(p.cfg));
         for (const auto& sh : shapes) {
-            std::vector<BatchPass> batch;
-            for (size_t k = 0; k < jobs.size(); ++k) {
-                if (key(plans[k].cfg) != sh) continue;
-                BatchPass bp;
-                bp.plan = &plans[k];
-                bp.dev = &devs[k];
-                bp.frames = jobs[k].d_frames;
-                bp.g0 = 0;
-                bp.g1 = static_cast<int>(plans[k].groups.size());
-                bp.max_snr = jobs[k].d_max;
-                bp.best_v = jobs[k].d_bv;
-                batch.push_back(bp);
-            }
+            batch.clear();
+            for (size_t k = 0; k < jobs.size(); ++k)
+                if (plans[k].stream.empty() && key(plans[k].cfg) == sh) batch.push_back(pass(k));
             DevBuf& desc = c.scratch(kDesc, batch_desc_bytes(static_cast<int>(batch.size())), "stack descriptors");
             stack_launch_batch(batch, desc.as<unsigned char>(), desc.bytes(), c.err_flag(), c.sms(), c.stream());
             ++c.launches;

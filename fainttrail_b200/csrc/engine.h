@@ -164,10 +164,10 @@ struct PassJob {
 // Plans built ahead on host threads: a pass's plan depends only on its shift
 // table, sizes and tile shape, so it can be made while the GPU still runs the
 // work queued before the stacking (the null runs' preprocessing). A pass whose
-// shape is not yet known (the autotuner has not timed its kind) gets none.
+// shape is not yet known (the autotuner has not timed its kind) gets an empty one.
 struct PlanAhead {
-    std::vector<std::shared_future<StackPlan>> plans;  // per job; invalid: none
-    std::vector<StackConfig> cfgs;                     // the configuration each plan is made for
+    std::vector<std::shared_future<StackPlan>> plans;  // per job; invalid: none; m = 0: left to the autotuner
+    int shape = 0;                                     // the process-wide tile shape they are made for
 };
 PlanAhead plan_ahead(Context& c, std::vector<PassJob> tables);
 

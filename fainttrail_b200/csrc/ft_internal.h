@@ -10,6 +10,8 @@
 #include <string>
 #include <vector>
 
+#include "stack_stream.h"
+
 namespace ftb {
 
 struct CudaError : std::runtime_error {
@@ -88,6 +90,9 @@ struct StackPlan {
     long long max_group_bytes = 0;            // largest windows + offset table of one group
     int max_slots = 0;
     double adds = 0;                          // m * n * w * h
+    // a streamed pass: its own tables (stack_stream.h), those above empty but inv_sqrt
+    StreamPlan stream;
+    int ngroups() const { return static_cast<int>(stream.empty() ? groups.size() : stream.groups.size()); }
 };
 
 // Motion blocks for the planner, flattened: kMotionBlock slots a block, -1 for a
@@ -101,7 +106,16 @@ std::vector<int> motion_order(const int* dx, const int* dy, int m, int n, double
 StackPlan make_stack_plan(int w, int h, int n, const int* dx, const int* dy, int m, int min_count,
                           const std::vector<int>& order, const StackConfig& cfg);
 
-StackConfig choose_stack_config(int w, int h, int n, int device_smem_optin);
+// The process-wide shape where its windows fit, else by frame count and by how
+// close the rows of the blocks of `order` are.
+StackConfig choose_stack_config(int n, const int* dx, const int* dy, const std::vector<int>& order,
+                                int device_smem_optin);
+
+// The streamed plan of a pass where `shape` asks for one (kStreamShape, or 0 and
+// the rule on its sizes) and its motions pack for it: `plan` and true, else false.
+// ahead: the plan is made while other passes run.
+bool make_streamed_pass(int w, int h, int n, const int* dx, const int* dy, int m, int min_count, int shape, bool ahead,
+                        StackPlan& plan);
 
 // The maps of a pass whose min_count exceeds its frame count, where no S/N is
 // defined: max_snr +0.0f and best_v -1 for `pixels` dense pixels.
@@ -119,9 +133,12 @@ void allow_dynamic_smem(const void* func, size_t bytes);
 
 // Compiled stack kernel shapes: 1 = 32 x 16 tiles (12 warps), 2 = 64 x 8 tiles with
 // paired columns (12 warps), 3 = 32 x 8 (16 warps), 4 = 32 x 4 (16 warps),
-// 5 = 32 x 16 with one shared maximum per tile (16 warps), 6 = the same with 14 warps,
+// 5 = 32 x 16 with one shared maximum per tile (16 warps), 6 = 32 x 16 with the
+// frames streamed past blocks of five motions (stack_stream.cu; a pass whose
+// motions do not pack for it takes the automatic choice among the others),
 // 7 = 32 x 12 (16 warps), 8 = 32 x 20 with the shared maximum (16 warps).
 constexpr int kStackShapes = 8;
+constexpr int kStreamShape = 6;
 StackConfig stack_shape_config(int shape, int device_smem_optin);
 bool stack_shape_fits(const StackConfig& c, int n);
 // A process-wide choice for choose_stack_config: 0 = by frame count, else a shape
@@ -133,9 +150,11 @@ int stack_shape();
 // wait_cycles clock cycles with the error flag set; 0 restores the normal
 // launches (no extra bytes, a two-second limit).
 void set_wait_test(int extra_bytes, long long wait_cycles);
+void wait_test(unsigned& extra_bytes, long long& wait_cycles);
 
-// Device copy of a plan.
+// Device copy of a plan, in one block.
 struct StackPlanDev {
+    void* block = nullptr;
     StackGroup* groups = nullptr;
     StackWin* wins = nullptr;
     int* slot_motion = nullptr;
@@ -143,6 +162,9 @@ struct StackPlanDev {
     int* slot_off_base = nullptr;
     short2* slot_shift = nullptr;
     float* inv_sqrt = nullptr;
+    StreamGroup* stream_groups = nullptr;
+    StreamWin* stream_wins = nullptr;
+    uint32_t* stream_desc = nullptr;
     int ngroups = 0;
     void upload(const StackPlan& p, cudaStream_t s);
     void release();
@@ -163,6 +185,7 @@ struct BatchPass {
     float* max_snr = nullptr;
     int* best_v = nullptr;
     int tile_rows0 = 0, tile_rows = 0;  // a band of tile rows only (0 rows: the whole pass)
+    unsigned long long* keys = nullptr; // streamed passes in parts: the maps' running maxima, w * h
 };
 
 // Device bytes of the descriptors of a batch (a work-queue counter, one tensor
@@ -174,5 +197,14 @@ size_t batch_desc_bytes(int npasses);
 // (cfg.ty, cfg.p). d_desc: device buffer of at least batch_desc_bytes bytes.
 void stack_launch_batch(const std::vector<BatchPass>& batch, unsigned char* d_desc, size_t desc_bytes, int* d_err,
                         int sms, cudaStream_t s);
+
+// Streamed passes in one persistent launch (plans with stream tables): a tile's
+// groups are cut into `splits` work items; a pass with splits above 1, or in
+// group ranges, merges its maxima in bp.keys. d_desc: stream_desc_bytes. Returns
+// the kernels launched.
+int stream_splits(const std::vector<const StackPlan*>& plans, int sms);
+size_t stream_desc_bytes(int npasses);
+int stream_launch(const std::vector<BatchPass>& batch, int splits, unsigned char* d_desc, size_t desc_bytes, int* d_err,
+                  int sms, cudaStream_t s);
 
 }  // namespace ftb

@@ -89,9 +89,14 @@ extern "C" int ft_b200_stack_dev_noalloc(const float* d_frames, int width, int h
             FTB_CHECK(cudaStreamSynchronize(s));
             return FT_B200_OK;
         }
-        const StackConfig cfg = choose_stack_config(width, height, nframes, d.smem_optin);
+        // the 32 x 16 tile where it fits: the table sizes that the array's limit was stated for
+        const std::vector<int> order = motion_order(dx, dy, motions, nframes, 4.0, 4.0);
+        StackConfig cfg = stack_shape_config(1, d.smem_optin);
+        if (!stack_shape_fits(cfg, nframes)) cfg = stack_shape_config(3, d.smem_optin);
+        if (stack_shape() != 0 || !stack_shape_fits(cfg, nframes))
+            cfg = choose_stack_config(nframes, dx, dy, order, d.smem_optin);
         StackPlan plan = make_stack_plan(width, height, nframes, dx, dy, motions, min_count,
-                                         motion_order(dx, dy, motions, nframes, 4.0, 4.0), cfg);
+                                         order, cfg);
         plan.pitch = pitch;
         // the plan tables, one after another at 256-byte boundaries in the array
         struct Part {

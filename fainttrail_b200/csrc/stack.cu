@@ -43,6 +43,7 @@
 #include <unordered_map>
 
 #include "ft_internal.h"
+#include "stack_device.cuh"
 
 namespace ftb {
 
@@ -188,6 +189,13 @@ std::vector<int> motion_order(const int* dx, const int* dy, int m, int n, double
 }
 
 namespace {
+// float(1 / sqrt(c)), c = 0..n (0 for none)
+std::vector<float> inverse_roots(int n) {
+    std::vector<float> v(static_cast<size_t>(n) + 1, 0.0f);
+    for (int c = 1; c <= n; ++c) v[static_cast<size_t>(c)] = static_cast<float>(1.0 / std::sqrt(static_cast<double>(c)));
+    return v;
+}
+
 inline int floor4(int v) { return (v >> 2) * 4; }  // arithmetic shift: floor for negatives too
 inline int roundup(int v, int q) { return (v + q - 1) / q * q; }
 }  // namespace
@@ -204,6 +212,11 @@ void set_wait_test(int extra_bytes, long long wait_cycles) {
         throw std::runtime_error("wait test: extra bytes in [0, 1 MiB] and a limit of at least 1000 cycles");
     g_wait_cycles = extra_bytes > 0 ? wait_cycles : 4000000000LL;
     g_wait_extra = extra_bytes;
+}
+
+void wait_test(unsigned& extra_bytes, long long& wait_cycles) {
+    extra_bytes = static_cast<unsigned>(g_wait_extra.load());
+    wait_cycles = extra_bytes > 0 ? g_wait_cycles.load() : 4000000000LL;
 }
 
 void set_stack_shape(int shape) {
@@ -227,10 +240,6 @@ StackConfig stack_shape_config(int shape, int smem_optin) {
             c.tile_w = 32; c.wp = 40; c.p = 16; c.ty = 16; c.merge = 1; c.rows = shape_row_spread(16, 1);
             c.smem_bytes -= 32 * 16 * 8;  // the keys sit ahead of the windows
             break;
-        case 6:  // the same with 14 warps (146 registers a thread)
-            c.tile_w = 32; c.wp = 40; c.p = 16; c.ty = 14; c.merge = 1; c.rows = shape_row_spread(16, 1);
-            c.smem_bytes -= 32 * 16 * 8;
-            break;
         case 7: c.tile_w = 32; c.wp = 40; c.p = 12; c.ty = 16; c.rows = shape_row_spread(12, 0); break;
         case 8:  // 32 x 20 with the shared maximum: 16 warps
             c.tile_w = 32; c.wp = 40; c.p = 20; c.ty = 16; c.merge = 1; c.rows = shape_row_spread(20, 1);
@@ -248,21 +257,97 @@ bool stack_shape_fits(const StackConfig& c, int n) {
     return need <= static_cast<long long>(c.smem_bytes) * 7 / 10;
 }
 
-StackConfig choose_stack_config(int w, int h, int n, int smem_optin) {
-    (void)w;
-    (void)h;
+namespace {
+
+constexpr int kShortRows = 24;
+// streamed against resident windows, kernel + plan in ms: 48 frames of 2048^2 78.4 +
+// 1.6 against 75.6 + 7.6, 56 of 2048 x 1024 49.5 + 2.1 against 50.2 + 9.3, 72: 99.5 +
+// 4.3 against 171 + 18, 120: 462 + 21 against 1080 + 97
+constexpr int kResidentFrames = 48;
+// 20 frames of 1024^2 10.4 + 0.8 against 8.9 + 3.0, of 2048^2 6.2 + 0.1 against 5.9 +
+// 0.5; 30 of 1024 x 768 24.9 + 2.4 against 22.7 + 10.5; 40 of 2048^2 46.4 + 0.9
+// against 42.4 + 4.3
+constexpr long long kStreamPixels = 2LL << 20;
+// kernels only: 30 frames of 256 x 192 2.2 against 3.6, of 512 x 384 7.4 against 8.2,
+// of 768 x 576 15.9 against 14.0
+constexpr long long kStreamPixelsAhead = 200000;
+
+}  // namespace
+
+// Whether most blocks keep to row offsets of 1, as the 32 x 12 and the
+// shared-maximum kernels take them (others are cut, and their rests padded): a
+// sample of blocks, every frame.
+static bool close_rows(int n, const int* dx, const int* dy, const std::vector<int>& order) {
+    constexpr size_t M = kMotionBlock;
+    const size_t nblk = order.size() / M, step = std::max<size_t>(1, nblk / 64);
+    size_t seen = 0, wide = 0;
+    for (size_t b = 0; b < nblk; b += step, ++seen) {
+        bool far = false;
+        for (int i = 0; i < n && !far; ++i) {
+            int lx = INT32_MAX, hx = INT32_MIN, ly = INT32_MAX, hy = INT32_MIN;
+            for (size_t k = 0; k < M; ++k) {
+                const int j = order[b * M + k];
+                if (j < 0) continue;
+                const size_t e = static_cast<size_t>(j) * n + static_cast<size_t>(i);
+                lx = std::min(lx, dx[e]);
+                hx = std::max(hx, dx[e]);
+                ly = std::min(ly, dy[e]);
+                hy = std::max(hy, dy[e]);
+            }
+            far = lx < hx || static_cast<long long>(hy) - ly > 1;
+        }
+        wide += far;
+    }
+    return wide * 10 <= seen;
+}
+
+StackConfig choose_stack_config(int n, const int* dx, const int* dy, const std::vector<int>& order, int smem_optin) {
     const int forced = g_shape;
-    if (forced > 0) {
+    if (forced > 0 && forced != kStreamShape) {
         const StackConfig c = stack_shape_config(forced, smem_optin);
         if (stack_shape_fits(c, n)) return c;
     }
-    // the first shape whose windows fit: single-column tiles of 16, 8 and 4 rows
-    // (taller frame stacks need the shorter tiles)
-    for (int s : {1, 3}) {
+    // The first whose windows fit. Motions close in rows: up to kShortRows frames
+    // 32 x 12, where the per-thread maxima cost less than the shared one (9 passes of
+    // 20 frames of 1024^2 74.4 ms; 32 x 16 with the shared maximum 75.7, with
+    // per-thread maxima 78.3; 12 frames of 1024 x 768 1.74 against 1.82 ms); then
+    // 32 x 16 with the shared maximum (33 frames of 2048^2 24.3 ms, 32 x 12 24.5,
+    // per-thread 25.6; 10 passes of 30 frames of 1024^2 268, 273 and 283 ms); then
+    // 32 x 12 to 62 frames (56 frames of 2048 x 1024 50.2 ms, 32 x 8 79.7). Other
+    // motions: 32 x 16 with per-thread maxima. Taller frame stacks need the shorter
+    // tiles.
+    const bool close = close_rows(n, dx, dy, order);
+    for (int s : {close ? (n <= kShortRows ? 7 : 5) : 1, close ? 7 : 3, 3}) {
         const StackConfig c = stack_shape_config(s, smem_optin);
         if (stack_shape_fits(c, n)) return c;
     }
     return stack_shape_config(4, smem_optin);
+}
+
+bool make_streamed_pass(int w, int h, int n, const int* dx, const int* dy, int m, int min_count, int shape, bool ahead,
+                        StackPlan& plan) {
+    // a byte a row counts a border pixel's frames
+    if ((shape != 0 && shape != kStreamShape) || w <= 0 || h <= 0 || n <= 0 || n > 255 || m <= 0 || min_count < 1)
+        return false;
+    // The automatic choice: above kResidentFrames, where a tile's windows of all
+    // frames leave shared memory room for few motions at once, and for images of up to
+    // kStreamPixels, where the cheaper plan and the tiles split over the SMs count;
+    // plans made ahead are hidden behind other work, so only the split counts there.
+    if (shape == 0 && n <= kResidentFrames &&
+        static_cast<long long>(w) * h > (ahead ? kStreamPixelsAhead : kStreamPixels))
+        return false;
+    plan = StackPlan();
+    plan.stream = make_stream_plan(w, h, n, dx, dy, m);
+    if (plan.stream.empty()) return false;
+    plan.w = w;
+    plan.h = h;
+    plan.n = n;
+    plan.m = m;
+    plan.min_count = min_count;
+    plan.pitch = frame_pitch(w);
+    plan.adds = static_cast<double>(m) * n * w * h;
+    plan.inv_sqrt = inverse_roots(n);
+    return true;
 }
 
 StackPlan make_stack_plan(int w, int h, int n, const int* dx, const int* dy, int m, int min_count,
@@ -284,8 +369,7 @@ StackPlan make_stack_plan(int w, int h, int n, const int* dx, const int* dy, int
     // shared memory in floats after the barrier and alignment slack
     const long long budget = (cfg.smem_bytes - 256) / 4;
 
-    P.inv_sqrt.assign(static_cast<size_t>(n) + 1, 0.0f);
-    for (int c = 1; c <= n; ++c) P.inv_sqrt[static_cast<size_t>(c)] = static_cast<float>(1.0 / std::sqrt(static_cast<double>(c)));
+    P.inv_sqrt = inverse_roots(n);
 
     // clamped shifts: beyond +-w / +-h a frame never covers, as within
     auto cdx = [&](int j, int i) { return std::clamp(dx[static_cast<size_t>(j) * n + i], -w, w); };
@@ -564,39 +648,57 @@ StackPlan make_stack_plan(int w, int h, int n, const int* dx, const int* dy, int
 
 void StackPlanDev::upload(const StackPlan& p, cudaStream_t s) {
     release();
+    // every table at a 256-byte boundary of one block, brought by one copy
+    std::vector<unsigned char> host;
+    std::vector<std::pair<void**, size_t>> at;
     auto put = [&](auto*& dst, const auto& v) {
-        using T = std::remove_reference_t<decltype(v[0])>;
-        const size_t bytes = std::max<size_t>(1, v.size()) * sizeof(T);
-        FTB_CHECK(cudaMallocAsync(reinterpret_cast<void**>(&dst), bytes, s));
-        if (!v.empty()) FTB_CHECK(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
+        using T = std::remove_cv_t<std::remove_reference_t<decltype(v[0])>>;
+        const size_t off = (host.size() + 255) / 256 * 256;
+        at.emplace_back(reinterpret_cast<void**>(&dst), off);
+        host.resize(off + std::max<size_t>(1, v.size()) * sizeof(T));
+        if (!v.empty()) std::memcpy(host.data() + off, v.data(), v.size() * sizeof(T));
     };
-    put(groups, p.groups);
-    put(wins, p.wins);
-    put(slot_motion, p.slot_motion);
-    put(slot_off, p.slot_off);
-    put(slot_off_base, p.slot_off_base);
-    put(slot_shift, p.slot_shift);
+    if (p.stream.empty()) {
+        put(groups, p.groups);
+        put(wins, p.wins);
+        put(slot_motion, p.slot_motion);
+        put(slot_off, p.slot_off);
+        put(slot_off_base, p.slot_off_base);
+        put(slot_shift, p.slot_shift);
+    } else {
+        put(stream_groups, p.stream.groups);
+        put(stream_wins, p.stream.wins);
+        put(stream_desc, p.stream.desc);
+        put(slot_motion, p.stream.slot_motion);
+    }
     put(inv_sqrt, p.inv_sqrt);
-    ngroups = static_cast<int>(p.groups.size());
+    FTB_CHECK(cudaMallocAsync(&block, host.size(), s));
     stream_ = s;
+    for (const auto& [dst, off] : at) *dst = static_cast<unsigned char*>(block) + off;
+    FTB_CHECK(cudaMemcpyAsync(block, host.data(), host.size(), cudaMemcpyHostToDevice, s));
+    ngroups = p.ngroups();
 }
 
 void StackPlanDev::release() {
-    for (void* q : {static_cast<void*>(groups), static_cast<void*>(wins), static_cast<void*>(slot_motion),
-                    static_cast<void*>(slot_off), static_cast<void*>(slot_off_base), static_cast<void*>(slot_shift),
-                    static_cast<void*>(inv_sqrt)})
-        if (q) cudaFreeAsync(q, stream_);
-    groups = nullptr;
-    wins = nullptr;
-    slot_motion = nullptr;
-    slot_off = nullptr;
-    slot_off_base = nullptr;
-    slot_shift = nullptr;
-    inv_sqrt = nullptr;
-    ngroups = 0;
+    if (block) cudaFreeAsync(block, stream_);
+    *this = StackPlanDev();
 }
 
 // ------------------------------------------------------------------ device
+
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+    });
+    if (!fn) throw CudaError("cuTensorMapEncodeTiled is not available from the driver");
+    return fn;
+}
 
 namespace {
 
@@ -621,63 +723,6 @@ struct StackArgs {
     unsigned extra_tx;      // bytes the staging barrier expects beyond its copies (0; a test of the bounded wait)
     long long wait_limit;   // clock cycles a staging wait may take
 };
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            smem_addr(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar))
-        : "memory");
-}
-
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// Bounded wait on the staging barrier: `limit` clock cycles (about two seconds
-// by default), then the kernel records an error and gives up (the host turns it
-// into an exception).
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* err, long long limit) {
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (clock64() - t0 > limit) {
-            atomicExch(err, 1);
-            return false;
-        }
-    }
-    return true;
-}
-
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
-        "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
 
 template <int P, int WP>
 __device__ __forceinline__ void load_column(float (&v)[P], const float* __restrict__ src) {
@@ -819,18 +864,6 @@ __device__ __forceinline__ void motion_quad(const StackArgs& a, const StackGroup
 // reference's rule. S/N is never -0.0 (sums start at +0.0f and round to
 // nearest) and -inf / NaN never enter, as in the register rule. Frees 2P
 // registers per thread, so 16-row tiles run 16 warps.
-
-__device__ __forceinline__ unsigned long long snr_key(float s, int j) {
-    const uint32_t b = __float_as_uint(s);
-    const uint32_t o = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-    return (static_cast<unsigned long long>(o) << 32) | static_cast<uint32_t>(~j);
-}
-
-__device__ __forceinline__ void snr_unkey(unsigned long long k, float& s, int& j) {
-    const uint32_t o = static_cast<uint32_t>(k >> 32);
-    s = __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-    j = static_cast<int>(~static_cast<uint32_t>(k));
-}
 
 // Pairs of floats: __fadd2_rn / __fmul2_rn are two independent
 // round-to-nearest operations per call, bit-identical to two scalar ones
@@ -1597,20 +1630,6 @@ __global__ void __launch_bounds__(32 * NW, 1)
     }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    });
-    if (!fn) throw CudaError("cuTensorMapEncodeTiled is not available from the driver");
-    return fn;
-}
-
 template <int NW, int P, int WP, int BH, int TW, int MERGE>
 void launch_batch(const std::vector<BatchPass>& batch, unsigned char* d_desc, size_t desc_bytes, int* d_err,
                   int sms, cudaStream_t s) {
@@ -1634,7 +1653,7 @@ void launch_batch(const std::vector<BatchPass>& batch, unsigned char* d_desc, si
                                        static_cast<cuuint64_t>(plan.pitch) * plan.h * 4};
         const cuuint32_t box[3] = {WP, BH, 1};
         const cuuint32_t estr[3] = {1, 1, 1};
-        const CUresult r = encode_fn()(&maps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(bp.frames), dims,
+        const CUresult r = tensor_map_encoder()(&maps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(bp.frames), dims,
                                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS)
@@ -1670,8 +1689,7 @@ void launch_batch(const std::vector<BatchPass>& batch, unsigned char* d_desc, si
         a.max_snr = bp.max_snr;
         a.best_v = bp.best_v;
         a.err = d_err;
-        a.extra_tx = static_cast<unsigned>(g_wait_extra.load());
-        a.wait_limit = g_wait_extra.load() > 0 ? g_wait_cycles.load() : 4000000000LL;
+        wait_test(a.extra_tx, a.wait_limit);
         smem = std::max(smem, 256 + keys_bytes + static_cast<size_t>(plan.max_group_bytes));
         if (smem > static_cast<size_t>(plan.cfg.smem_bytes) + 256 + keys_bytes)
             throw std::runtime_error("stack plan exceeds shared memory");
@@ -1708,8 +1726,6 @@ void stack_launch_batch(const std::vector<BatchPass>& batch, unsigned char* d_de
         launch_batch<16, 4, 40, 4, 32, 0>(batch, d_desc, desc_bytes, d_err, sms, s);
     else if (c.tile_w == 32 && c.wp == 40 && c.ty == 16 && c.p == 16 && c.merge == 1)
         launch_batch<16, 16, 40, 4, 32, 1>(batch, d_desc, desc_bytes, d_err, sms, s);
-    else if (c.tile_w == 32 && c.wp == 40 && c.ty == 14 && c.p == 16 && c.merge == 1)
-        launch_batch<14, 16, 40, 4, 32, 1>(batch, d_desc, desc_bytes, d_err, sms, s);
     else if (c.tile_w == 32 && c.wp == 40 && c.ty == 16 && c.p == 12 && c.merge == 0)
         launch_batch<16, 12, 40, 4, 32, 0>(batch, d_desc, desc_bytes, d_err, sms, s);
     else if (c.tile_w == 32 && c.wp == 40 && c.ty == 16 && c.p == 20 && c.merge == 1)

@@ -102,7 +102,7 @@ int ft_b200_stack_dev_noalloc(const float* d_frames, int width, int height, int 
 /* One stacking pass computed on the host exactly as the device kernel computes
  * it, for checks of the pass planner on a machine without a GPU (the role of the
  * reference's emulate_cuda_pass, cuda_plan.cpp:74-117): the pass is planned for
- * kernel shape `shape` (1..7 as ft_b200_set_tile_shape; 0: the automatic choice)
+ * kernel shape `shape` (1..8 as ft_b200_set_tile_shape; 0: the automatic choice)
  * with a B200's 227 KB of shared memory per block, and the plan -- tiles, motion
  * groups, frame windows zero-filled outside the frame, 16-bit window offsets,
  * coverage counts with the interior-tile shortcut, float adds in ascending frame
@@ -416,21 +416,24 @@ int ft_b200_check_registration_dev(ft_b200_ctx* ctx, const float* d_frames, int 
 int ft_b200_result_registration(const ft_b200_result* r, ft_b200_drift_check* out);
 
 /* Stack kernel tile shape for every later pass in this process: 0 = automatic
- * (the default: the autotuned choice where one is cached for the pass's frame
- * count, else the first shape whose windows fit), 1 = 32 x 16 output tiles,
- * 2 = 64 x 8 tiles with paired columns, 3 = 32 x 8, 4 = 32 x 4, 5 and 6 = 32 x 16
- * with one shared maximum per tile (16 and 14 warps), 7 = 32 x 12, 8 = 32 x 20
- * with the shared maximum (16 warps). A fixed shape
- * whose frame windows do not fit shared memory falls back to automatic. Results
+ * (the default: by frame count and size; among the shapes other than 6 the
+ * autotuned choice where one is cached), 1 = 32 x 16 output tiles,
+ * 2 = 64 x 8 tiles with paired columns, 3 = 32 x 8, 4 = 32 x 4, 5 = 32 x 16
+ * with one shared maximum per tile, 6 = 32 x 16 with the frames streamed past the
+ * motions, 7 = 32 x 12, 8 = 32 x 20 with the shared maximum. A fixed shape
+ * whose frame windows do not fit shared memory, or 6 for motions that do not pack
+ * into blocks of five with one column and at most one row step, falls back to
+ * automatic. Results
  * do not depend on the shape. No counterpart in the reference (its CUDA kernel
  * has one shape, backend_cuda.cu:55-72). */
 int ft_b200_set_tile_shape(int shape);
 int ft_b200_tile_shape(void);
 /* The autotuner's choices so far: for a pass of at least 5e11 adds whose
- * (frames, motions, width, height) it has not seen, automatic mode plans every
- * shape that fits, times each on a band of tile rows in the middle of the image
+ * (frames, motions, width, height) it has not seen, and that is not streamed (6), automatic mode plans
+ * every other shape that fits, times each on a band of tile rows in the middle of the image
  * and keeps the fastest per output pixel. Fills keys[4 * k .. 4 * k + 3] (frames,
- * motions, width, height) and shapes[k] for up to cap entries; returns the count.
+ * motions, width, height) and shapes[k] (6 for a streamed pass of that size) for
+ * up to cap entries; returns the count.
  * ft_b200_clear_tuned_shapes forgets them. */
 int ft_b200_tuned_shapes(int* keys, int* shapes, int cap);
 void ft_b200_clear_tuned_shapes(void);
