@@ -384,39 +384,73 @@ __global__ void __launch_bounds__(64) sky_net_kernel(const SkyArgs a) {
 
 // The regular sample grid of sample_pixels (common.hpp:85-100): every step-th
 // column and row from `border`, finite values only, optionally masked. Order is
-// irrelevant (only order statistics are taken); the count is exact.
-__global__ void sample_kernel(const float* img, size_t plane, int w, int h, int pitch, int n, int border, int step,
-                              int gw, int gh, const float* mask, float* out, int cap, int* counts) {
-    const int f = blockIdx.y;
-    const long long g = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (g >= static_cast<long long>(gw) * gh) return;
-    const int x = border + static_cast<int>(g % gw) * step, y = border + static_cast<int>(g / gw) * step;
-    const size_t pix = static_cast<size_t>(y) * pitch + x;
-    if (mask && mask[pix] == 0.0f) return;
-    const float v = img[f * plane + pix];
-    if (!finitef(v)) return;
-    const int k = atomicAdd(&counts[f], 1);
-    if (k < cap) out[static_cast<size_t>(f) * cap + k] = v;
+// irrelevant (only order statistics are taken); the count is exact. The image may
+// be a band of a larger one: it holds the rows from oy on (row y at img + (y - oy) *
+// pitch), and the grid is the whole image's, its rows border + (j0 + j) step for j <
+// gh.
+//
+// Bound by memory, once the frame's counter is taken once for a CTA's 2048 points
+// (one atomic a warp before: sampling and selection together 4.8 ms for 120 frames of
+// 1030 x 777, now 0.95 ms).
+constexpr int kSamplePoints = 8;  // of a thread
+
+__global__ void __launch_bounds__(256) sample_kernel(const float* img, size_t plane, int pitch, int border, int step, int gw,
+                                                     int j0, int gh, int oy, const float* mask, float* out, int cap,
+                                                     int* counts) {
+    __shared__ int warp_first[8];
+    __shared__ int first;
+    const int f = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned points = static_cast<unsigned>(gw) * static_cast<unsigned>(gh);  // at most 4 x 200000 (grid_step)
+    const unsigned g0 = blockIdx.x * (256u * kSamplePoints) + threadIdx.x;
+    float v[kSamplePoints];
+    unsigned ok = 0;
+#pragma unroll
+    for (int i = 0; i < kSamplePoints; ++i) {
+        const unsigned g = g0 + 256u * i;
+        v[i] = CUDART_NAN_F;
+        if (g < points) {
+            const unsigned row = g / static_cast<unsigned>(gw);
+            const int x = border + static_cast<int>(g - row * gw) * step;
+            const int y = border + (j0 + static_cast<int>(row)) * step - oy;
+            const size_t pix = static_cast<size_t>(y) * pitch + x;
+            if (!mask || mask[pix] != 0.0f) v[i] = img[f * plane + pix];
+        }
+    }
+    int mine = 0, before = 0;  // of this warp: its samples, and this thread's first
+#pragma unroll
+    for (int i = 0; i < kSamplePoints; ++i) {
+        const unsigned b = __ballot_sync(0xffffffffu, finitef(v[i]));
+        if (b >> lane & 1u) ok |= 1u << i;
+        mine += __popc(b);
+    }
+    if (lane == 0) warp_first[warp] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+        for (int k = 0; k < 8; ++k) {
+            const int c = warp_first[k];
+            warp_first[k] = sum;
+            sum += c;
+        }
+        first = sum ? atomicAdd(&counts[f], sum) : 0;
+    }
+    __syncthreads();
+    before = first + warp_first[warp];
+#pragma unroll
+    for (int i = 0; i < kSamplePoints; ++i) {
+        const unsigned b = __ballot_sync(0xffffffffu, ok >> i & 1u);
+        const int k = before + __popc(b & ((1u << lane) - 1u));
+        if ((ok >> i & 1u) && k < cap) out[static_cast<size_t>(f) * cap + k] = v[i];
+        before += __popc(b);
+    }
 }
 
-// sample_kernel for a band of a larger image: the band holds image rows
-// [oy, oy + rows) (row y at img + (y - oy) * pitch); the grid is the whole
-// image's (columns border + i step, rows border + (j0 + j) step for the gh grid
-// rows inside the band's core), so the samples are those the whole image gives
-// in those rows.
-__global__ void sample_band_kernel(const float* img, size_t plane, int pitch, int n, int border, int step, int gw,
-                                   int j0, int gh, int oy, const float* mask, float* out, int cap, int* counts) {
-    const int f = blockIdx.y;
-    const long long g = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (g >= static_cast<long long>(gw) * gh) return;
-    const int x = border + static_cast<int>(g % gw) * step;
-    const int y = border + (j0 + static_cast<int>(g / gw)) * step - oy;
-    const size_t pix = static_cast<size_t>(y) * pitch + x;
-    if (mask && mask[pix] == 0.0f) return;
-    const float v = img[f * plane + pix];
-    if (!finitef(v)) return;
-    const int k = atomicAdd(&counts[f], 1);
-    if (k < cap) out[static_cast<size_t>(f) * cap + k] = v;
+inline void launch_sample(const float* img, size_t plane, int pitch, int n, int border, int step, int gw, int j0, int gh,
+                          int oy, const float* mask, float* out, int cap, int* counts, cudaStream_t s) {
+    const long long g = static_cast<long long>(gw) * gh, each = 256 * kSamplePoints;
+    sample_kernel<<<dim3(static_cast<unsigned>((g + each - 1) / each), n), 256, 0, s>>>(img, plane, pitch, border, step, gw,
+                                                                                      j0, gh, oy, mask, out, cap, counts);
+    FTB_CHECK(cudaGetLastError());
 }
 
 __device__ __forceinline__ uint32_t order_key(float v) {
@@ -427,99 +461,241 @@ __device__ __forceinline__ float key_value(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// k-th smallest key (0-based) of the CTA's values, by four 8-bit radix passes.
-// MODE 0: keys of x; MODE 1: keys of float(|x - med|) (the MAD deviations,
-// common.hpp:80). Needs >= 256 threads.
-// ---- exact order statistics of a frame's samples by a cluster of CTAs: four
-// 8-bit radix passes over order-preserving keys; each CTA counts its share of
-// the samples into its own histogram, CTA 0 merges the cluster's histograms
-// through distributed shared memory and picks the digit, and a cluster barrier
-// separates the passes (eight SMs per frame).
+// ---- exact order statistics of a frame's samples by a cluster of CTAs.
+//
+// The samples near the wanted rank are copied into shared memory, and radix passes
+// over them (11 bits each, of the range that is left) find the value. Which are near
+// comes from 1024 samples at regular places: the values 64 ranks on either side of
+// theirs (four standard deviations of a random subset's) hold it, and an eighth of
+// all samples. One pass over the samples then counts those below and collects those
+// between. Where that misses (few distinct values overfill the lists, or an unlucky
+// subset), the radix passes read all samples. Up to kSelAll samples are all kept.
+//
+// Bound by reading the samples once a median (two a sigma): an 8-bit radix select
+// over all of them for either middle rank, 16 passes a sigma and most of their
+// shared atomics on one of a few exponents' counters, measured 2.9 ms for 120 frames
+// of 790,000 samples; sampling and this 4.8 ms then, 0.95 ms now.
 
 namespace cg = cooperative_groups;
 constexpr int kSelCluster = 8;
+constexpr int kSelThreads = 512;
+constexpr int kSelList = 16384;  // keys a CTA keeps
+constexpr int kSelBits = 11;
+constexpr int kSelSubset = 1024;
+constexpr int kSelSlack = 64;  // subset ranks on either side
+constexpr int kSelAll = kSelCluster * kSelList;
 
+struct SelShared {
+    uint32_t list[kSelList];
+    uint32_t hist[2][1 << kSelBits];
+    uint32_t subset[kSelSubset];
+    uint32_t bracket[2];
+    int count, below;  // of this CTA: keys inside the bracket, below it
+    uint32_t low;      // largest key below the result
+    uint32_t warp_sum[kSelThreads / 32];
+    uint32_t digit, before;
+    int total[3];      // of the cluster: inside, below; whether a list overflowed
+};
+
+// MODE 0: keys of x; MODE 1: keys of float(|x - med|) (the MAD deviations,
+// common.hpp:80).
 template <int MODE>
-__device__ uint32_t cluster_select(const float* x, int cnt, int k, double med, uint32_t* hist, uint32_t* merged,
-                                   uint32_t* res) {
-    cg::cluster_group cl = cg::this_cluster();
-    const unsigned rank = cl.block_rank();
-    const int stride = static_cast<int>(blockDim.x) * kSelCluster;
-    uint32_t prefix = 0, pmask = 0;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
-        cl.sync();  // no CTA still reads a histogram of the previous pass
-        for (int e = static_cast<int>(rank * blockDim.x + threadIdx.x); e < cnt; e += stride) {
-            float v = x[e];
-            if (MODE == 1) v = __double2float_rn(fabs(static_cast<double>(v) - med));
-            const uint32_t key = order_key(v);
-            if ((key & pmask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-        }
-        cl.sync();
-        if (rank == 0) {
-            for (int b = threadIdx.x; b < 256; b += blockDim.x) {
-                uint32_t sum = 0;
-                for (int r = 0; r < kSelCluster; ++r) sum += cl.map_shared_rank(hist, r)[b];
-                merged[b] = sum;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                uint32_t acc = 0;
-                int d = 0;
-                for (; d < 255; ++d) {
-                    if (acc + merged[d] > static_cast<uint32_t>(k)) break;
-                    acc += merged[d];
-                }
-                res[0] = static_cast<uint32_t>(d);
-                res[1] = acc;
-            }
-        }
-        cl.sync();
-        const uint32_t* r0 = cl.map_shared_rank(res, 0);
-        const uint32_t d = r0[0];
-        k -= static_cast<int>(r0[1]);
-        prefix |= d << shift;
-        pmask |= 255u << shift;
-    }
-    cl.sync();  // CTA 0's result is read before it is overwritten
-    return prefix;
+__device__ __forceinline__ uint32_t sample_key(float v, double med) {
+    if (MODE == 1) v = __double2float_rn(fabs(static_cast<double>(v) - med));
+    return order_key(v);
 }
 
+// The median of cnt > 0 values, in every thread of the cluster: the value of rank
+// cnt / 2 or, for an even count, its mean with the one before (common.hpp:64-76).
 template <int MODE>
-__device__ double cluster_median(const float* x, int cnt, double med, uint32_t* hist, uint32_t* merged, uint32_t* res) {
-    if (cnt == 0) return 0.0;
+__device__ double cluster_median(const float* __restrict__ x, int cnt, double med, SelShared& sh) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = static_cast<int>(cl.block_rank()), t = static_cast<int>(threadIdx.x), lane = t & 31, warp = t >> 5;
     const int mid = cnt / 2;
-    double m = key_value(cluster_select<MODE>(x, cnt, mid, med, hist, merged, res));
-    if (cnt % 2 == 0) {
-        const float lower = key_value(cluster_select<MODE>(x, cnt, mid - 1, med, hist, merged, res));
+    const bool even = cnt % 2 == 0;
+    uint32_t lo = 0u, hi = 0xffffffffu;
+    if (t == 0) {
+        sh.count = sh.below = 0;
+        sh.low = 0u;
+    }
+    for (int b = t; b < 2 << kSelBits; b += kSelThreads) sh.hist[0][b] = 0u;  // both
+    if (cnt > kSelAll) {
+        for (int q = t; q < kSelSubset; q += kSelThreads)
+            sh.subset[q] = sample_key<MODE>(x[static_cast<long long>(q) * cnt / kSelSubset], med);
+        __syncthreads();
+        // the ranks of an eighth of the subset, four threads a value
+        const int q = rank * (kSelSubset / kSelCluster) + (t >> 2);
+        const uint32_t own = sh.subset[q];
+        int r = 0;
+        for (int e = t & 3; e < kSelSubset; e += 4) r += sh.subset[e] < own || (sh.subset[e] == own && e < q);
+        r += __shfl_xor_sync(0xffffffffu, r, 1);
+        r += __shfl_xor_sync(0xffffffffu, r, 2);
+        const int mine = r == kSelSubset / 2 - kSelSlack ? 0 : r == kSelSubset / 2 + kSelSlack ? 1 : -1;
+        if (mine >= 0 && (t & 3) == 0)
+            for (int c = 0; c < kSelCluster; ++c) *cl.map_shared_rank(&sh.bracket[mine], c) = own;
+        cl.sync();
+        lo = sh.bracket[0];
+        hi = sh.bracket[1];
+    } else {
+        __syncthreads();
+    }
+    // the keys between go to the list, those below are counted
+    constexpr int kUnroll = 4;
+    int below = 0;
+    for (int e0 = rank * kSelThreads; e0 < cnt; e0 += kSelThreads * kSelCluster * kUnroll) {
+        float v[kUnroll];
+#pragma unroll
+        for (int i = 0; i < kUnroll; ++i) {
+            const int e = e0 + i * kSelThreads * kSelCluster + t;
+            v[i] = e < cnt ? x[e] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < kUnroll; ++i) {
+            const bool valid = e0 + i * kSelThreads * kSelCluster + t < cnt;
+            const uint32_t key = sample_key<MODE>(v[i], med);
+            below += valid && key < lo;
+            const bool in = valid && key >= lo && key <= hi;
+            const unsigned b = __ballot_sync(0xffffffffu, in);
+            if (b) {
+                int first = 0;
+                if (lane == 0) first = atomicAdd(&sh.count, __popc(b));
+                first = __shfl_sync(0xffffffffu, first, 0) + __popc(b & ((1u << lane) - 1u));
+                if (in && first < kSelList) sh.list[first] = key;
+            }
+        }
+    }
+    below = __reduce_add_sync(0xffffffffu, below);
+    if (lane == 0 && below) atomicAdd(&sh.below, below);
+    cl.sync();
+    if (warp == 0) {
+        int inside = 0, under = 0, over = 0;
+        if (lane < kSelCluster) {
+            inside = *cl.map_shared_rank(&sh.count, lane);
+            under = *cl.map_shared_rank(&sh.below, lane);
+            over = inside > kSelList;
+        }
+        inside = __reduce_add_sync(0xffffffffu, inside);
+        under = __reduce_add_sync(0xffffffffu, under);
+        over = __reduce_add_sync(0xffffffffu, over);
+        if (lane == 0) {
+            sh.total[0] = inside;
+            sh.total[1] = under;
+            sh.total[2] = over;
+        }
+    }
+    __syncthreads();
+    int k = mid - sh.total[1];  // rank among the keys that are looked at
+    const bool listed = sh.total[2] == 0 && k - even >= 0 && k < sh.total[0];
+    if (!listed) {
+        lo = 0u;
+        hi = 0xffffffffu;
+        k = mid;
+    }
+    const int own = listed ? sh.count : 0;
+    auto each = [&](auto&& f) {
+        if (listed) {
+            for (int e = t; e < own; e += kSelThreads) f(sh.list[e]);
+        } else {
+            for (int e = rank * kSelThreads + t; e < cnt; e += kSelThreads * kSelCluster) f(sample_key<MODE>(x[e], med));
+        }
+    };
+    // radix passes over the keys in [base, base + 2^bits). Each counts into one
+    // histogram and clears the other: a pass's are read after its barrier, and all
+    // CTAs have read them when the next one's barrier is passed.
+    uint32_t base = lo;
+    int bits = 32 - __clz(hi - lo), flip = 0;
+    while (bits > 0) {
+        const int shift = max(0, bits - kSelBits);
+        const uint32_t span = bits < 32 ? (1u << bits) - 1u : 0xffffffffu;
+        uint32_t* hist = sh.hist[flip];
+        each([&](uint32_t key) {
+            const uint32_t d = key - base;
+            if (key >= base && d <= span) atomicAdd(&hist[d >> shift], 1u);
+        });
+        cl.sync();
+        // four digits a thread, summed over the cluster, and the one that holds rank k
+        uint32_t sum[4] = {};
+#pragma unroll
+        for (int c = 0; c < kSelCluster; ++c) {
+            const uint4 h = reinterpret_cast<const uint4*>(cl.map_shared_rank(hist, c))[t];
+            sum[0] += h.x;
+            sum[1] += h.y;
+            sum[2] += h.z;
+            sum[3] += h.w;
+        }
+        const uint32_t all = sum[0] + sum[1] + sum[2] + sum[3];
+        uint32_t acc = all;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, acc, o);
+            if (lane >= o) acc += up;
+        }
+        if (lane == 31) sh.warp_sum[warp] = acc;
+        __syncthreads();
+        for (int q = 0; q < warp; ++q) acc += sh.warp_sum[q];
+        acc -= all;
+        const uint32_t want = static_cast<uint32_t>(k);
+        if (want >= acc && want < acc + all) {
+            int d = 0;
+            while (d < 3 && want >= acc + sum[d]) acc += sum[d++];
+            sh.digit = static_cast<uint32_t>(4 * t + d);
+            sh.before = acc;
+        }
+        flip ^= 1;
+        for (int b = t; b < 1 << kSelBits; b += kSelThreads) sh.hist[flip][b] = 0u;
+        __syncthreads();
+        base += sh.digit << shift;
+        k -= static_cast<int>(sh.before);
+        bits = shift;
+    }
+    double m = key_value(base);
+    if (even) {
+        float lower = key_value(base);
+        if (k == 0) {  // no equal one before: the largest key below
+            uint32_t top = 0u;
+            each([&](uint32_t key) {
+                if (key < base) top = max(top, key);
+            });
+            top = __reduce_max_sync(0xffffffffu, top);
+            if (lane == 0) atomicMax(&sh.low, top);
+            cl.sync();
+            for (int c = 0; c < kSelCluster; ++c) top = max(top, *cl.map_shared_rank(&sh.low, c));
+            lower = key_value(top);
+        }
         m = 0.5 * (m + lower);
     }
+    cl.sync();  // all is read before the next median, or the end, takes the memory
     return m;
 }
 
-// robust_sigma_kernel with a cluster of kSelCluster CTAs per frame
-__global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(256)
-    robust_sigma_cluster_kernel(const float* samples, int cap, const int* counts, double* out, int unit_if_zero) {
-    __shared__ uint32_t hist[256], merged[256], res[2];
+// sigma, or the median itself (MEDIAN), of a frame's samples: a cluster a frame
+template <bool MEDIAN>
+__global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(kSelThreads)
+    select_kernel(const float* samples, int cap, const int* counts, double* out, int unit_if_zero) {
+    extern __shared__ __align__(16) unsigned char sel[];
+    SelShared& sh = *reinterpret_cast<SelShared*>(sel);
     const int f = blockIdx.x / kSelCluster;
     const int cnt = min(counts[f], cap);
     const float* x = samples + static_cast<size_t>(f) * cap;
-    double sg = 0.0;
-    if (cnt >= 3) {
-        const double med = cluster_median<0>(x, cnt, 0.0, hist, merged, res);
-        sg = 1.4826 * cluster_median<1>(x, cnt, med, hist, merged, res);
+    double r = 0.0;
+    if (MEDIAN) {
+        if (cnt > 0) r = cluster_median<0>(x, cnt, 0.0, sh);
+    } else {
+        if (cnt >= 3) {
+            const double med = cluster_median<0>(x, cnt, 0.0, sh);
+            r = 1.4826 * cluster_median<1>(x, cnt, med, sh);
+        }
+        if (unit_if_zero && !(r > 0.0)) r = 1.0;
     }
-    if (cg::this_cluster().block_rank() == 0 && threadIdx.x == 0) out[f] = (unit_if_zero && !(sg > 0.0)) ? 1.0 : sg;
+    if (cg::this_cluster().block_rank() == 0 && threadIdx.x == 0) out[f] = r;
 }
 
-// median_kernel with a cluster per frame
-__global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(256)
-    median_cluster_kernel(const float* samples, int cap, const int* counts, double* out) {
-    __shared__ uint32_t hist[256], merged[256], res[2];
-    const int f = blockIdx.x / kSelCluster;
-    const int cnt = min(counts[f], cap);
-    const double m = cluster_median<0>(samples + static_cast<size_t>(f) * cap, cnt, 0.0, hist, merged, res);
-    if (cg::this_cluster().block_rank() == 0 && threadIdx.x == 0) out[f] = m;
+template <bool MEDIAN>
+inline void launch_select(const float* samples, int cap, const int* counts, int n, double* out, int unit_if_zero,
+                          cudaStream_t s) {
+    allow_dynamic_smem(reinterpret_cast<const void*>(select_kernel<MEDIAN>), sizeof(SelShared));
+    select_kernel<MEDIAN><<<n * kSelCluster, kSelThreads, sizeof(SelShared), s>>>(samples, cap, counts, out, unit_if_zero);
+    FTB_CHECK(cudaGetLastError());
 }
 
 // ------------------------------------------------------------------ scatter + mask
@@ -1179,16 +1355,11 @@ void stage_noise(Context& c, StageScratch& sc, const float* d_sub, int w, int h,
         const int st = grid_step(w, h, 2, 200000);
         if (st > 0) {
             const int gw = grid_count(2, w - 2, st), gh = grid_count(2, h - 2, st);
-            const long long g = static_cast<long long>(gw) * gh;
-            sample_kernel<<<dim3(static_cast<unsigned>((g + 255) / 256), n), 256, 0, s>>>(
-                sc.residual.as<float>(), plane, w, h, pitch, n, 2, st, gw, gh, nullptr, sc.samples.as<float>(), sc.cap,
-                tb.counts);
-            FTB_CHECK(cudaGetLastError());
-        ++c.launches;
+            launch_sample(sc.residual.as<float>(), plane, pitch, n, 2, st, gw, 0, gh, 0, nullptr, sc.samples.as<float>(),
+                          sc.cap, tb.counts, s);
+            ++c.launches;
         }
-        robust_sigma_cluster_kernel<<<n * kSelCluster, 256, 0, s>>>(sc.samples.as<float>(), sc.cap, tb.counts,
-                                                                     tb.sigma, 1);
-        FTB_CHECK(cudaGetLastError());
+        launch_select<false>(sc.samples.as<float>(), sc.cap, tb.counts, n, tb.sigma, 1, s);
         ++c.launches;
         c.span_end(span);
     }
@@ -1264,16 +1435,12 @@ void stage_filter(Context& c, StageScratch& sc, int w, int h, int n, const Stage
         const int st = grid_step(w, h, fb, 200000);
         if (st > 0) {
             const int gw = grid_count(fb, w - fb, st), gh = grid_count(fb, h - fb, st);
-            const long long g = static_cast<long long>(gw) * gh;
             if (static_cast<long long>(gw) * gh > sc.cap) throw std::runtime_error("stage: sample buffer too small");
-            sample_kernel<<<dim3(static_cast<unsigned>((g + 255) / 256), n), 256, 0, s>>>(
-                d_filtered, plane, w, h, pitch, n, fb, st, gw, gh, d_mask, sc.samples.as<float>(), sc.cap, d_counts);
-            FTB_CHECK(cudaGetLastError());
-        ++c.launches;
+            launch_sample(d_filtered, plane, pitch, n, fb, st, gw, 0, gh, 0, d_mask, sc.samples.as<float>(), sc.cap,
+                          d_counts, s);
+            ++c.launches;
         }
-        robust_sigma_cluster_kernel<<<n * kSelCluster, 256, 0, s>>>(sc.samples.as<float>(), sc.cap, d_counts, d_sg,
-                                                                     0);
-        FTB_CHECK(cudaGetLastError());
+        launch_select<false>(sc.samples.as<float>(), sc.cap, d_counts, n, d_sg, 0, s);
         ++c.launches;
         rescale_kernel<<<dim3(static_cast<unsigned>((npix + 255) / 256), n), 256, 0, s>>>(d_filtered, plane, w, h, pitch,
                                                                                        d_sg);
@@ -1307,15 +1474,11 @@ void prepare_sub(Context& c, StageScratch& sc, float* d_raw, float* d_sub, int w
     const int st = grid_step(w, h, 0, 200000);
     if (st > 0) {
         const int gw = grid_count(0, w, st), gh = grid_count(0, h, st);
-        const long long g = static_cast<long long>(gw) * gh;
-        sample_kernel<<<dim3(static_cast<unsigned>((g + 255) / 256), n), 256, 0, s>>>(
-            d_raw, plane, w, h, pitch, n, 0, st, gw, gh, nullptr, sc.samples.as<float>(), sc.cap, tb.counts);
-        FTB_CHECK(cudaGetLastError());
+        launch_sample(d_raw, plane, pitch, n, 0, st, gw, 0, gh, 0, nullptr, sc.samples.as<float>(), sc.cap, tb.counts, s);
         ++c.launches;
     }
-    median_cluster_kernel<<<n * kSelCluster, 256, 0, s>>>(sc.samples.as<float>(), sc.cap, tb.counts, tb.sg);
-    FTB_CHECK(cudaGetLastError());
-        ++c.launches;
+    launch_select<true>(sc.samples.as<float>(), sc.cap, tb.counts, n, tb.sg, 0, s);
+    ++c.launches;
     const dim3 grid(static_cast<unsigned>((npix + 255) / 256), n);
     subtract_kernel<<<grid, 256, 0, s>>>(d_raw, plane, w, h, pitch, tb.sg);
     FTB_CHECK(cudaGetLastError());
@@ -1365,24 +1528,18 @@ void sample_band(Context& c, const float* d_img, size_t plane, int pitch, int n,
     const int j1 = (hi - border + st - 1) / st;
     const int gh = j1 - j0;
     if (gh <= 0 || gw <= 0) return;
-    const long long g = static_cast<long long>(gw) * gh;
-    sample_band_kernel<<<dim3(static_cast<unsigned>((g + 255) / 256), n), 256, 0, c.stream()>>>(
-        d_img, plane, pitch, n, border, st, gw, j0, gh, oy, d_mask, d_samples, cap, d_counts);
-    FTB_CHECK(cudaGetLastError());
+    launch_sample(d_img, plane, pitch, n, border, st, gw, j0, gh, oy, d_mask, d_samples, cap, d_counts, c.stream());
     ++c.launches;
 }
 
 void select_sigma(Context& c, const float* d_samples, int cap, const int* d_counts, int n, double* d_out,
                   int unit_if_zero) {
-    robust_sigma_cluster_kernel<<<n * kSelCluster, 256, 0, c.stream()>>>(d_samples, cap, d_counts, d_out,
-                                                                          unit_if_zero);
-    FTB_CHECK(cudaGetLastError());
+    launch_select<false>(d_samples, cap, d_counts, n, d_out, unit_if_zero, c.stream());
     ++c.launches;
 }
 
 void select_median(Context& c, const float* d_samples, int cap, const int* d_counts, int n, double* d_out) {
-    median_cluster_kernel<<<n * kSelCluster, 256, 0, c.stream()>>>(d_samples, cap, d_counts, d_out);
-    FTB_CHECK(cudaGetLastError());
+    launch_select<true>(d_samples, cap, d_counts, n, d_out, 0, c.stream());
     ++c.launches;
 }
 
@@ -1393,9 +1550,7 @@ void sample_frames(Context& c, const float* d_frames, size_t plane, int pitch, i
     const int gw = grid_count(border, w - border, st), gh = grid_count(border, h - border, st);
     const long long g = static_cast<long long>(gw) * gh;
     if (g > cap) throw std::runtime_error("sample_frames: sample buffer too small");
-    sample_kernel<<<dim3(static_cast<unsigned>((g + 255) / 256), n), 256, 0, c.stream()>>>(
-        d_frames, plane, w, h, pitch, n, border, st, gw, gh, nullptr, d_samples, cap, d_counts);
-    FTB_CHECK(cudaGetLastError());
+    launch_sample(d_frames, plane, pitch, n, border, st, gw, 0, gh, 0, nullptr, d_samples, cap, d_counts, c.stream());
     ++c.launches;
 }
 
@@ -1483,19 +1638,14 @@ void frame_sample_stats(Context& c, const float* const* d_frames, int k, int w, 
         const long long g = static_cast<long long>(gw) * gh;
         if (g > cap) throw std::runtime_error("frame_sample_stats: sample buffer too small");
         for (int i = 0; i < k; ++i) {
-            sample_kernel<<<dim3(static_cast<unsigned>((g + 255) / 256), 1), 256, 0, s>>>(
-                d_frames[i], 0, w, h, pitch, 1, 0, st, gw, gh, nullptr, d_samples + static_cast<size_t>(i) * cap, cap,
-                d_counts + i);
-            FTB_CHECK(cudaGetLastError());
+            launch_sample(d_frames[i], 0, pitch, 1, 0, st, gw, 0, gh, 0, nullptr, d_samples + static_cast<size_t>(i) * cap,
+                          cap, d_counts + i, s);
             ++c.launches;
         }
     }
-    median_cluster_kernel<<<k * kSelCluster, 256, 0, s>>>(d_samples, cap, d_counts, d_stats);
-    FTB_CHECK(cudaGetLastError());
-    ++c.launches;
-    robust_sigma_cluster_kernel<<<k * kSelCluster, 256, 0, s>>>(d_samples, cap, d_counts, d_stats + k, 0);
-    FTB_CHECK(cudaGetLastError());
-    ++c.launches;
+    launch_select<true>(d_samples, cap, d_counts, k, d_stats, 0, s);
+    launch_select<false>(d_samples, cap, d_counts, k, d_stats + k, 0, s);
+    c.launches += 2;
 }
 
 }  // namespace ftb

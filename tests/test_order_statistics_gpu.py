@@ -1,0 +1,34 @@
+"""Frame statistics on the B200 where their selection changes its way: sample
+counts below and above what a cluster's lists hold, distributions with few distinct
+values (which overfill them), missing samples, two samples or none. The stage's
+sigmas and filtered frames equal the oracle's bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def values(kind, rng, shape):
+    v = rng.normal(0, 10, shape)
+    if kind == "coarse":  # a handful of distinct values
+        v = np.round(v / 12.0)
+    elif kind == "constant":
+        v = np.full(shape, 3.0)
+        v[..., ::97] = rng.normal(0, 1, v[..., ::97].shape)
+    elif kind == "ramp":  # values in image order
+        v = np.cumsum(np.abs(v), axis=-1) * rng.choice([-1, 1], shape[:-1] + (1,))
+    elif kind == "missing":
+        v[rng.random(shape) < 0.31] = np.nan
+    return v.astype(np.float32)
+
+
+@pytest.mark.parametrize("kind", ["normal", "coarse", "constant", "ramp", "missing"])
+@pytest.mark.parametrize("w,h", [(5, 5), (7, 5), (64, 41), (369, 359), (369, 366), (890, 890), (1203, 700)])
+def test_sigma(device, oracle, w, h, kind):
+    rng = np.random.default_rng(w * h)
+    sub = values(kind, rng, (5, h, w))
+    sub[1, : h // 2] = np.nan
+    t = np.linspace(-0.2, 0.2, 5)
+    got, want = device.stage(sub, t, 1.5), oracle.build_stage(sub, t, 1.5)
+    for k in ("sigma", "filtered"):
+        assert np.array_equal(np.asarray(got[k]), np.asarray(want[k]), equal_nan=True), k
