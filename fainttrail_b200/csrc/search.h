@@ -107,8 +107,8 @@ double median_of(std::vector<float> v);  // median_inplace (common.hpp:64-74)
 
 // ---- device steps
 // prepare_core's background and blank-border growth (preprocess.cpp:572-580,
-// 233-254): d_raw (overwritten) -> d_sub; per-frame backgrounds to h_bg.
-void prepare_sub(Context& c, StageScratch& sc, float* d_raw, float* d_sub, int w, int h, int n, double* h_bg);
+// 233-254): d_raw -> d_sub; per-frame backgrounds to h_bg.
+void prepare_sub(Context& c, StageScratch& sc, const float* d_raw, float* d_sub, int w, int h, int n, double* h_bg);
 // local maxima of a detection map above `floor` (search.cpp:105-131), in
 // raster order
 std::vector<Peak> device_peaks(Context& c, const float* d_max, const int* d_best_v, int w, int h, float floor,

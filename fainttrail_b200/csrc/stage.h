@@ -75,7 +75,7 @@ void select_sigma(Context& c, const float* d_samples, int cap, const int* d_coun
                   int unit_if_zero);
 void select_median(Context& c, const float* d_samples, int cap, const int* d_counts, int n, double* d_out);
 // background subtraction with per-frame backgrounds (device) and blank growth by 3
-void subtract_grow(Context& c, float* d_raw, float* d_sub, int w, int rows, int n, const double* d_bg);
+void subtract_grow(Context& c, const float* d_raw, float* d_sub, int w, int rows, int n, const double* d_bg);
 // scatter, mask and matched filter of sc.residual with the noise given (device);
 // with d_sg, normalised by it, else left unnormalised
 void stage_filter_given(Context& c, StageScratch& sc, int w, int rows, int n, const StageParams& sp,
