@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "engine.h"
@@ -79,82 +80,6 @@ __device__ __forceinline__ int nth_set_bit(uint32_t x, int k) {
     if (k >= c) { k -= c; pos += 2; x >>= 2; }
     if (k >= static_cast<int>(x & 1u)) pos += 1;
     return pos;
-}
-
-// Position of the k-th (0-based) set bit of a 64-bit x, k < popc(x): the
-// half that holds it by one population count, then nth_set_bit.
-__device__ __forceinline__ int nth_set_bit64(uint64_t x, int k) {
-    const uint32_t lo = static_cast<uint32_t>(x);
-    const int c = __popc(lo);
-    const bool up = k >= c;
-    return (up ? 32 : 0) + nth_set_bit(up ? static_cast<uint32_t>(x >> 32) : lo, up ? k - c : k);
-}
-
-// sky_finish for at most 64 W64 frames: the kept sorted positions (set:
-// outside the exclusion window) in W64 64-bit words (1 or 2), the lo-th by
-// population counts (nth_set_bit64 within its word) and the hi-th, when it
-// differs, as the next set bit above it.
-template <int W64>
-__device__ __forceinline__ void sky_finish_words(const SkyArgs& a, const float* V, const float* S,
-                                                 const unsigned char* PF, int T, int t, int m_all, size_t pix,
-                                                 size_t plane) {
-    static_assert(W64 == 1 || W64 == 2, "one or two words");
-    const int n = a.n, e = a.exclude;
-    // global median: the two middle floats are added in float (preprocess.cpp:171)
-    const float mid_sum = __fadd_rn(S[((m_all - 1) / 2) * T + t], S[(m_all / 2) * T + t]);
-    const double global = 0.5 * static_cast<double>(mid_sum);
-    a.sky[pix] = __double2float_rn(global);
-    uint64_t k0 = m_all >= 64 ? ~0ull : (1ull << m_all) - 1ull;
-    uint64_t k1 = W64 == 1 || m_all <= 64 ? 0ull : (m_all >= 128 ? ~0ull : (1ull << (m_all - 64)) - 1ull);
-    int m = m_all;
-    // flips position p (255: a non-finite value, none); d: the change in m
-    auto flip = [&](int p, int d) {
-        if (p == 255) return;
-        const uint64_t b = 1ull << (p & 63);
-        if (W64 == 1 || p < 64)
-            k0 ^= b;
-        else
-            k1 ^= b;
-        m += d;
-    };
-    if (e > 0)
-        for (int r = 0; r <= min(e, n - 1); ++r) flip(PF[r * T + t], -1);  // rank 0's window
-    for (int r = 0; r < n; ++r) {
-        if (e > 0 && r > 0) {
-            if (r - 1 - e >= 0) flip(PF[(r - 1 - e) * T + t], 1);  // leaves the window: kept again
-            if (r + e < n) flip(PF[(r + e) * T + t], -1);          // enters: excluded
-        }
-        const float v = V[r * T + t];
-        float* out = a.residual + a.frame_of[r] * plane + pix;
-        if (v == CUDART_INF_F) {
-            *out = CUDART_NAN_F;
-            continue;
-        }
-        double st = global;
-        if (e > 0 && m >= 5) {
-            const int lo = (m - 1) / 2, hi = m / 2;
-            int plo, phi;
-            if (W64 == 1) {
-                plo = nth_set_bit64(k0, lo);
-                phi = hi == lo ? plo : plo + __ffsll(static_cast<long long>(k0 >> (plo + 1)));
-            } else {
-                const int c0 = __popcll(k0);
-                plo = lo < c0 ? nth_set_bit64(k0, lo) : 64 + nth_set_bit64(k1, lo - c0);
-                if (hi == lo) {
-                    phi = plo;
-                } else if (hi < c0) {  // the next kept position is in the first word
-                    phi = plo + __ffsll(static_cast<long long>(k0 >> (plo + 1)));
-                } else if (lo < c0) {  // plo is the first word's last: the second word's first
-                    phi = 63 + __ffsll(static_cast<long long>(k1));
-                } else {
-                    phi = plo + __ffsll(static_cast<long long>(k1 >> (plo - 63)));
-                }
-            }
-            // double add of the two middle values (preprocess.cpp:198)
-            st = 0.5 * (static_cast<double>(S[plo * T + t]) + static_cast<double>(S[phi * T + t]));
-        }
-        *out = __double2float_rn(static_cast<double>(v) - st);
-    }
 }
 
 // The static sky and the leave-out residuals of one pixel from its values by
@@ -276,108 +201,302 @@ __global__ void __launch_bounds__(64) sky_kernel(const SkyArgs a) {
             PF[(e0 + b) * T + t] = fin ? static_cast<unsigned char>(pos[b]) : 255;
         }
     }
-    if constexpr (W <= 2)
-        sky_finish_words<1>(a, V, S, PF, T, t, m_all, pix, plane);
-    else
-        sky_finish<W>(a, V, S, PF, T, t, m_all, pix, plane);
+    sky_finish<W>(a, V, S, PF, T, t, m_all, pix, plane);
 }
 
-// The same for n <= N <= 128 with the sorted order from a bitonic network in
-// registers instead of counting ranks: the pixel's values (non-finite ones as
-// +inf) are sorted with float min / max, which orders everything but the two
-// zeros; where a -0.0 is present the zero run is rewritten with the zeros in
-// time-rank order, which is the reference's order of equal (value, rank) pairs.
-// Each rank's sorted position is then the lower bound of its value in the
-// sorted values plus the number of equal values of lower rank.
-template <int N>
-__global__ void __launch_bounds__(64) sky_net_kernel(const SkyArgs a) {
-    constexpr int W = (N + 31) / 32;
-    extern __shared__ unsigned char sm[];
-    const int T = blockDim.x, t = threadIdx.x;
-    const int n = a.n;
-    float* V = reinterpret_cast<float*>(sm);                            // [n][T] values by time rank, +inf if not finite
-    float* S = V + n * T;                                               // [n][T] finite values in sorted order
-    unsigned char* PF = reinterpret_cast<unsigned char*>(S + n * T);    // [n][T] sorted position by rank, 255: none
-    const long long q = static_cast<long long>(blockIdx.x) * T + t;
-    const int x = static_cast<int>(q % a.w), y = static_cast<int>(q / a.w);
-    if (y >= a.h) return;
+// ---- the same for n <= N <= 128, without sorted positions for all values
+//
+// Leaving out x of the m sorted values moves the median's position by at most x, so
+// with windows of at most X ranks every median lies at the sorted positions [(m - X -
+// 1) / 2, (m + X) / 2], about a quarter of them at the default window. The values are
+// sorted by a network in registers (Batcher's merge exchange), those middle ones kept
+// in shared memory, and a window's content is the number of its values below them and
+// a bitmask of the middle positions it takes. Equal values are interchangeable: one
+// that enters takes the first free position from its run's first on, one that leaves
+// frees the run's first taken one; where a run reaches beyond the middle, its
+// count says which part the next one belongs to. Only the two zeros are equal and
+// differ: where the pixel holds a -0.0 and a median's value is zero, the wanted one is
+// looked up in rank order.
+//
+// Bound by issue, mostly of the integer and compare pipe: 173 instructions a value at
+// 40 frames (a third of them in the loop over the ranks) where counting every rank
+// against all others and finishing on full masks took 330. 40 frames of 2048^2: 1.71
+// -> 1.02 ms; 120 of 1030 x 777 (a bitonic network, 64 threads a CTA with all
+// positions in shared memory): 5.46 -> 1.45 ms; 33 of 1501 x 1117: 0.57 -> 0.35 ms.
+
+// Masks: position of the lowest set bit (x != 0), of the k-th (0-based) set bit (k <
+// popc(x), x below 2^16 where small), and bit c, or 0 for a c beyond the mask.
+__device__ __forceinline__ int low_bit(uint32_t x) { return __ffs(static_cast<int>(x)) - 1; }
+__device__ __forceinline__ int low_bit(uint64_t x) { return __ffsll(static_cast<long long>(x)) - 1; }
+__device__ __forceinline__ int low_bit(unsigned __int128 x) {
+    const uint64_t lo = static_cast<uint64_t>(x);
+    return lo ? low_bit(lo) : 64 + low_bit(static_cast<uint64_t>(x >> 64));
+}
+__device__ __forceinline__ int nth_bit(uint32_t x, int k, bool small) {
+    int pos = 0;
+    if (!small) {
+        const int c = __popc(x & 0xffffu);
+        if (k >= c) { k -= c; pos = 16; x >>= 16; }
+    }
+    int c = __popc(x & 0xffu);
+    if (k >= c) { k -= c; pos += 8; x >>= 8; }
+    c = __popc(x & 0xfu);
+    if (k >= c) { k -= c; pos += 4; x >>= 4; }
+    c = __popc(x & 0x3u);
+    if (k >= c) { k -= c; pos += 2; x >>= 2; }
+    return pos + (k >= static_cast<int>(x & 1u));
+}
+__device__ __forceinline__ int nth_bit(uint64_t x, int k, bool) {
+    const uint32_t lo = static_cast<uint32_t>(x);
+    const int c = __popc(lo);
+    const bool up = k >= c;
+    return (up ? 32 : 0) + nth_bit(up ? static_cast<uint32_t>(x >> 32) : lo, up ? k - c : k, false);
+}
+__device__ __forceinline__ int nth_bit(unsigned __int128 x, int k, bool) {
+    const uint64_t lo = static_cast<uint64_t>(x);
+    const int c = __popcll(lo);
+    const bool up = k >= c;
+    return (up ? 64 : 0) + nth_bit(up ? static_cast<uint64_t>(x >> 64) : lo, up ? k - c : k, false);
+}
+__device__ __forceinline__ void one_bit(uint32_t& x, unsigned c) { asm("shl.b32 %0, 1, %1;" : "=r"(x) : "r"(c)); }
+__device__ __forceinline__ void one_bit(uint64_t& x, unsigned c) { asm("shl.b64 %0, 1, %1;" : "=l"(x) : "r"(c)); }
+__device__ __forceinline__ void one_bit(unsigned __int128& x, unsigned c) {
+    x = c < 128u ? static_cast<unsigned __int128>(1) << c : 0;
+}
+
+// A rank's code: in its low bits its run's first middle position, or none (the masks'
+// one_bit gives 0), or a run that reaches beyond the middle (equal to its first value;
+// to its last, and not the first); above them, signed, what its exclusion adds to u =
+// kept values - 2 (kept values below the middle): 0 for a non-finite value, 1 below the
+// middle, else -1. The median's lower position is the (u - 1) / 2-th kept one of the
+// middle.
+template <class Mask>
+struct SkyCode {
+    using type = short;
+    static constexpr int bits = 9;
+};
+template <>
+struct SkyCode<uint32_t> {
+    using type = signed char;
+    static constexpr int bits = 6;
+};
+
+__host__ __device__ constexpr int sky_threads(int N) { return N <= 64 ? 128 : 64; }
+// Positions of the middle at most, for a window of 2 exclude + 1 ranks, and the rows
+// that a halving search over them reads (2^k - 1).
+__host__ __device__ inline int sky_middle(int n, int exclude) {
+    const int x = exclude < n ? 2 * exclude + 1 : n;
+    return x + 2 < n ? x + 2 : n;
+}
+__host__ __device__ inline int sky_rows(int middle) {
+    int r = 1;
+    while (r < middle) r = 2 * r + 1;
+    return r;
+}
+
+template <int N, class Mask>
+__global__ void __launch_bounds__(sky_threads(N)) sky_middle_kernel(const SkyArgs a) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    using Code = typename SkyCode<Mask>::type;
+    constexpr int T = sky_threads(N), kBits = SkyCode<Mask>::bits;
+    constexpr int kNone = (1 << kBits) - 1, kFirst = kNone - 1, kLast = kNone - 2;
+    constexpr int kBelow = 1 << kBits, kOther = -(1 << kBits);
+    // frames that are there for certain: launch_sky takes the smallest network
+    constexpr int kSure = sizeof(Mask) > 4 ? 0 : N <= 64 ? N - 8 : N - 16;
+    constexpr bool kHeld = N <= 64;  // the values stay in shared memory; more are read again
+    const int t = threadIdx.x, n = a.n, e = min(a.exclude, n), most = sky_middle(n, e), rows = sky_rows(most);
+    size_t* at = reinterpret_cast<size_t*>(sm);       // [n] a rank's frame, from the first pixel
+    float* S = reinterpret_cast<float*>(at + n) + t;  // [rows][T] the middle values, then +inf
+    float* V = S + rows * T;                          // [n][T] values by time rank, +inf if not finite
+    // [n + 2 e + 1][T] by time rank, from rank -e - 1 on: none outside the sequence
+    Code* code = reinterpret_cast<Code*>(S - t + T * (rows + (kHeld ? n : 0))) + t + T * (e + 1);
     const size_t plane = static_cast<size_t>(a.pitch) * a.h;
+    for (int r = t; r < n; r += T) at[r] = a.frame_of[r] * plane;
+    __syncthreads();
+    const unsigned q = blockIdx.x * static_cast<unsigned>(T) + t;
+    const int y = static_cast<int>(q / static_cast<unsigned>(a.w)), x = static_cast<int>(q - y * static_cast<unsigned>(a.w));
+    if (y >= a.h) return;
     const size_t pix = static_cast<size_t>(y) * a.pitch + x;
+    const float* sub = a.sub + pix;
+    float* residual = a.residual + pix;
     float sv[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) sv[r] = r < kSure || r < n ? __ldg(sub + at[r]) : CUDART_INF_F;
     int m_all = 0;
     bool negzero = false;
 #pragma unroll
     for (int r = 0; r < N; ++r) {
-        float v = CUDART_INF_F;
-        if (r < n) {
-            const float u = a.sub[a.frame_of[r] * plane + pix];
-            const bool fin = finitef(u);
-            v = fin ? u : CUDART_INF_F;
-            m_all += fin;
-            negzero |= __float_as_uint(u) == 0x80000000u;
-            V[r * T + t] = v;
-        }
-        sv[r] = v;
+        if (!finitef(sv[r])) sv[r] = CUDART_INF_F;
+        m_all += sv[r] != CUDART_INF_F;
+        negzero |= __float_as_uint(sv[r]) == 0x80000000u;
+        if (kHeld && (r < kSure || r < n)) V[r * T] = sv[r];
     }
     if (m_all < a.need) {
         a.sky[pix] = CUDART_NAN_F;
-        for (int i = 0; i < n; ++i) a.residual[i * plane + pix] = CUDART_NAN_F;
+        for (int i = 0; i < n; ++i) residual[i * plane] = CUDART_NAN_F;
         return;
     }
+    auto value = [&](int r) {
+        if (kHeld) return V[r * T];
+        const float v = sub[at[r]];
+        return finitef(v) ? v : CUDART_INF_F;
+    };
 #pragma unroll
-    for (int k = 2; k <= N; k <<= 1)
+    for (int p = 1; p < N; p <<= 1)
 #pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1)
+        for (int k = p; k > 0; k >>= 1)
 #pragma unroll
-            for (int i = 0; i < N; ++i) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const float lo = fminf(sv[i], sv[l]), hi = fmaxf(sv[i], sv[l]);
-                    if ((i & k) == 0) {
-                        sv[i] = lo;
-                        sv[l] = hi;
-                    } else {
-                        sv[i] = hi;
-                        sv[l] = lo;
-                    }
+            for (int i = 0; i < N; ++i)
+                if (i >= k % p && i + k < N && ((i - k % p) / k) % 2 == 0 && i / (2 * p) == (i + k) / (2 * p)) {
+                    const float lo = fminf(sv[i], sv[i + k]), hi = fmaxf(sv[i], sv[i + k]);
+                    sv[i] = lo;
+                    sv[i + k] = hi;
                 }
-            }
+    // the middle: positions [first, first + len)
+    const int X = e < n ? min(2 * e + 1, n) : n;
+    const int first = max(0, (m_all - X - 1) >> 1), len = min(m_all - 1, (m_all + X) >> 1) - first + 1;
+    {
+        float* to = S - first * T;
 #pragma unroll
-    for (int p = 0; p < N; ++p)
-        if (p < m_all) S[p * T + t] = sv[p];
-    if (negzero) {
-        int p = 0;
-        while (p < m_all && S[p * T + t] < 0.0f) ++p;
-        for (int r = 0; r < n; ++r) {
-            const float v = V[r * T + t];
-            if (v == 0.0f) S[(p++) * T + t] = v;
-        }
+        for (int p = 0; p < N; ++p)
+            if (p >= first && p < first + len) to[p * T] = sv[p];
+        for (int p = len; p < rows; ++p) S[p * T] = CUDART_INF_F;
     }
-    for (int r = 0; r < n; ++r) {
-        const float v = V[r * T + t];
-        if (v == CUDART_INF_F) {
-            PF[r * T + t] = 255;
-            continue;
+    // the k-th value (0-based) in (value, time rank) order outside the window of rank r
+    // (r < -e: no window), which is a zero
+    auto zero = [&](int k, int r) {
+        for (int i = 0; i < n; ++i)
+            if (abs(i - r) > e) k -= value(i) < 0.0f;
+        float z = 0.0f;
+        for (int i = 0; i < n && k >= 0; ++i)
+            if (abs(i - r) > e && value(i) == 0.0f) {
+                z = value(i);
+                --k;
+            }
+        return z;
+    };
+    auto middle = [&](int pos, int k, int r) {
+        const float v = S[pos * T];
+        return negzero && v == 0.0f ? zero(k, r) : v;
+    };
+    // global median: the two middle floats are added in float (preprocess.cpp:171)
+    const int far = -2 * n - e;
+    const double global = 0.5 * static_cast<double>(__fadd_rn(middle((m_all - 1) / 2 - first, (m_all - 1) / 2, far),
+                                                              middle(m_all / 2 - first, m_all / 2, far)));
+    a.sky[pix] = __double2float_rn(global);
+    if (e <= 0) {
+        for (int r = 0; r < n; ++r) {
+            const float v = value(r);
+            residual[at[r]] = v != CUDART_INF_F ? __double2float_rn(static_cast<double>(v) - global) : CUDART_NAN_F;
         }
-        int lo = 0, len = m_all;
-        while (len > 0) {
-            const int half = len >> 1;
-            if (S[(lo + half) * T + t] < v) {
-                lo += half + 1;
-                len -= half + 1;
-            } else {
-                len = half;
+        return;
+    }
+    auto lower_bound = [&](float v) {
+        int p = 0;
+#pragma unroll
+        for (int s = 4 * static_cast<int>(sizeof(Mask)); s > 0; s >>= 1)
+            if (s < rows + 1 && S[(p + s - 1) * T] < v) p += s;
+        return p;
+    };
+    // runs that reach beyond the middle's ends: values of the first below it, and where
+    // the last one's starts
+    int run_below, run_last = 0;
+    bool runs;
+    {
+        const float s0 = S[0], s1 = S[(len - 1) * T];
+        int less = 0, upto = 0;  // values below the first, up to the last
+#pragma unroll 4
+        for (int r = 0; r < n; ++r) {
+            const float v = value(r);
+            const int p = lower_bound(v);
+            const bool below = v < s0;
+            less += below;
+            upto += v <= s1;
+            const int c = below ? kNone + kBelow : v <= s1 ? p + kOther : v != CUDART_INF_F ? kNone + kOther : kNone;
+            code[r * T] = static_cast<Code>(c);
+        }
+        run_below = first - less;
+        const bool beyond = upto > first + len;
+        runs = run_below > 0 || beyond;
+        if (runs) {
+            run_last = lower_bound(s1);
+            for (int r = 0; r < n; ++r) {
+                const float v = value(r);
+                if (v == s0 && (run_below > 0 || s0 == s1))
+                    code[r * T] = static_cast<Code>(kFirst + kOther);
+                else if (v == s1 && beyond)
+                    code[r * T] = static_cast<Code>(kLast + kOther);
             }
         }
-        int p = lo;
-        if (lo + 1 < m_all && S[(lo + 1) * T + t] == v)
-            for (int f = 0; f < r; ++f) p += V[f * T + t] == v;
-        PF[r * T + t] = static_cast<unsigned char>(p);
     }
-    if constexpr (N <= 128)
-        sky_finish_words<(N + 63) / 64>(a, V, S, PF, T, t, m_all, pix, plane);
+    for (int r = 1; r <= e + 1; ++r) code[-r * T] = static_cast<Code>(kNone);
+    for (int r = n; r < n + e; ++r) code[r * T] = static_cast<Code>(kNone);
+    Mask out = 0;                     // middle positions in the window
+    int u = m_all - 2 * first;        // kept values - 2 (kept ones below the middle)
+    int first_out = 0, last_out = 0;  // excluded ones of the runs beyond the middle's ends
+    const Mask all = len >= static_cast<int>(8 * sizeof(Mask)) ? ~static_cast<Mask>(0) : (static_cast<Mask>(1) << len) - 1;
+    // the position that such a run's next excluded (d = 1) or included (-1) value takes
+    auto in_run = [&](int c, int d) {
+        if (c == kFirst) {
+            const int k = d > 0 ? first_out : first_out - 1;
+            first_out += d;
+            if (k < run_below) u += 2 * d;
+            return k >= run_below && k < run_below + len ? 0 : kNone;
+        }
+        const int k = d > 0 ? last_out : last_out - 1;
+        last_out += d;
+        return k < len - run_last ? run_last : kNone;
+    };
+    auto enter = [&](int c, bool runs) {
+        u += c >> kBits;
+        c &= kNone;
+        if (runs && (c == kFirst || c == kLast)) c = in_run(c, 1);
+        Mask bit;
+        one_bit(bit, static_cast<unsigned>(c));
+        out |= out + bit;
+    };
+    auto leave = [&](int c, bool runs) {
+        u -= c >> kBits;
+        c &= kNone;
+        if (runs && (c == kFirst || c == kLast)) c = in_run(c, -1);
+        Mask bit;
+        one_bit(bit, static_cast<unsigned>(c));
+        const Mask up = out & (~bit + 1);
+        out ^= up & (~up + 1);
+    };
+    for (int r = 0; r < e; ++r) enter(r < n ? code[r * T] : kNone, runs);
+    auto finish = [&](auto kind) {  // plain: no runs beyond the middle, no -0.0, five values kept always
+        constexpr bool kPlain = decltype(kind)::value;
+        int m = m_all;
+        if (!kPlain)
+            for (int r = 0; r < min(e, n); ++r) m -= value(r) != CUDART_INF_F;
+#pragma unroll 2
+        for (int r = 0; r < n; ++r) {
+            leave(code[(r - 1 - e) * T], !kPlain && runs);
+            enter(code[(r + e) * T], !kPlain && runs);
+            const float v = value(r);
+            double st = global;
+            if (!kPlain) m += (r - 1 - e >= 0 && value(r - 1 - e) != CUDART_INF_F) - (r + e < n && value(r + e) != CUDART_INF_F);
+            if (kPlain || m >= 5) {
+                const Mask kept = all & ~out;
+                const int plo = nth_bit(kept, (u - 1) >> 1, rows <= 15);
+                const Mask above = kept & ~((static_cast<Mask>(2) << plo) - 1);
+                const int phi = u & 1 ? plo : low_bit(above);
+                float s0 = S[plo * T], s1 = S[phi * T];
+                if (!kPlain && negzero) {
+                    s0 = middle(plo, (m - 1) >> 1, r);
+                    s1 = middle(phi, m >> 1, r);
+                }
+                // double add of the two middle values (preprocess.cpp:198)
+                st = 0.5 * (static_cast<double>(s0) + static_cast<double>(s1));
+            }
+            residual[at[r]] = v != CUDART_INF_F ? __double2float_rn(static_cast<double>(v) - st) : CUDART_NAN_F;
+        }
+    };
+    if (runs || negzero || a.need - X < 5)
+        finish(std::false_type());
     else
-        sky_finish<W>(a, V, S, PF, T, t, m_all, pix, plane);
+        finish(std::true_type());
 }
 
 // ------------------------------------------------------------------ samples + exact medians
@@ -963,13 +1082,50 @@ __global__ void __launch_bounds__(256) filter_kernel(const FilterArgs a) {
 // the static sky: counted ranks up to 64 frames (measured faster there: 554
 // against 375 GB/s at 40 frames), the sorting network up to 128 (where the
 // counting grows with n^2), counted ranks beyond
-void launch_sky(const SkyArgs& a, int n, long long npix, cudaStream_t s) {
-    const int T = 64;
-    const size_t smem = static_cast<size_t>(T) * n * 9;
-    auto kern = n <= 64 ? sky_kernel<2> : n <= 128 ? sky_net_kernel<128> : sky_kernel<8>;
+template <int N, class Mask>
+void launch_sky_middle(const SkyArgs& a, long long npix, cudaStream_t s) {
+    constexpr int T = sky_threads(N);
+    const size_t smem = sizeof(size_t) * a.n + static_cast<size_t>(T) *
+        (4 * sky_rows(sky_middle(a.n, a.exclude)) + ((N <= 64 ? 4 : 0) + sizeof(typename SkyCode<Mask>::type)) * a.n +
+         sizeof(typename SkyCode<Mask>::type) * (2 * std::min(a.exclude, a.n) + 1));
+    auto kern = sky_middle_kernel<N, Mask>;
     allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
     kern<<<static_cast<unsigned>((npix + T - 1) / T), T, smem, s>>>(a);
     FTB_CHECK(cudaGetLastError());
+}
+
+// Up to 128 frames the sort is a network of the next multiple of 8 or 16 values and the
+// middle's mask the smallest that holds it (a longer window than the default one may
+// need 64 or 128 bits, which only the 64- and 128-value networks are compiled for);
+// more frames: rank counting.
+void launch_sky(const SkyArgs& a, int n, long long npix, cudaStream_t s) {
+    const int middle = sky_middle(n, a.exclude);
+    if (n > 128 || npix > 0x7fffffffLL) {
+        const int T = 64;
+        const size_t smem = static_cast<size_t>(T) * n * 9;
+        allow_dynamic_smem(reinterpret_cast<const void*>(sky_kernel<8>), smem);
+        sky_kernel<8><<<static_cast<unsigned>((npix + T - 1) / T), T, smem, s>>>(a);
+        FTB_CHECK(cudaGetLastError());
+    } else if (middle > 64) {
+        launch_sky_middle<128, unsigned __int128>(a, npix, s);
+    } else if (middle > 32) {
+        n <= 64 ? launch_sky_middle<64, uint64_t>(a, npix, s) : launch_sky_middle<128, uint64_t>(a, npix, s);
+    } else {
+        switch (n <= 64 ? (n + 7) / 8 : 8 + (n - 64 + 15) / 16) {
+            case 1: launch_sky_middle<8, uint32_t>(a, npix, s); break;
+            case 2: launch_sky_middle<16, uint32_t>(a, npix, s); break;
+            case 3: launch_sky_middle<24, uint32_t>(a, npix, s); break;
+            case 4: launch_sky_middle<32, uint32_t>(a, npix, s); break;
+            case 5: launch_sky_middle<40, uint32_t>(a, npix, s); break;
+            case 6: launch_sky_middle<48, uint32_t>(a, npix, s); break;
+            case 7: launch_sky_middle<56, uint32_t>(a, npix, s); break;
+            case 8: launch_sky_middle<64, uint32_t>(a, npix, s); break;
+            case 9: launch_sky_middle<80, uint32_t>(a, npix, s); break;
+            case 10: launch_sky_middle<96, uint32_t>(a, npix, s); break;
+            case 11: launch_sky_middle<112, uint32_t>(a, npix, s); break;
+            default: launch_sky_middle<128, uint32_t>(a, npix, s); break;
+        }
+    }
 }
 
 // the temporal scatter: the sorting network up to 128 frames, counting beyond

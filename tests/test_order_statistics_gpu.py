@@ -32,3 +32,24 @@ def test_sigma(device, oracle, w, h, kind):
     got, want = device.stage(sub, t, 1.5), oracle.build_stage(sub, t, 1.5)
     for k in ("sigma", "filtered"):
         assert np.array_equal(np.asarray(got[k]), np.asarray(want[k]), equal_nan=True), k
+
+
+@pytest.mark.parametrize("n", [5, 8, 9, 40, 63, 65, 97, 113, 128])
+def test_windows(device, oracle, n):
+    """Leave-out windows from none to the whole sequence on values with long runs of
+    equal ones, signed zeros and missing values."""
+    rng = np.random.default_rng(n)
+    sub = rng.integers(-2, 3, (n, 7, 65)).astype(np.float32)
+    sub[:, 1] = rng.normal(0, 1, (n, 65))
+    sub[:, 2] = 1.0
+    sub[sub == 0] = rng.choice(np.array([0.0, -0.0], np.float32), np.count_nonzero(sub == 0))
+    sub[rng.random(sub.shape) < 0.2] = np.nan
+    sub[:, 4:, :20] = np.round(rng.normal(0, 40, (n, 3, 20)))
+    t = rng.permutation(np.linspace(-0.3, 0.3, n))
+    for exclude in (0, 1, 2, n // 8, 15, 16, 31, 32, n // 2, n - 1, n, 10 * n):
+        got = device.stage(sub, t, 1.5, static_exclude=exclude)
+        want = oracle.build_stage(sub, t, 1.5, static_exclude=exclude)
+        for k in ("static_sky", "filtered", "sigma"):
+            a, b = np.asarray(got[k]), np.asarray(want[k])
+            assert np.array_equal(a, b, equal_nan=True), (exclude, k)
+            assert np.array_equal(np.signbit(a[a == 0]), np.signbit(b[b == 0])), (exclude, k)
