@@ -53,3 +53,19 @@ def test_windows(device, oracle, n):
             a, b = np.asarray(got[k]), np.asarray(want[k])
             assert np.array_equal(a, b, equal_nan=True), (exclude, k)
             assert np.array_equal(np.signbit(a[a == 0]), np.signbit(b[b == 0])), (exclude, k)
+
+
+@pytest.mark.parametrize("n", [5, 8, 17, 40, 64, 65, 100, 128, 131])
+@pytest.mark.parametrize("decades", [0.0, 3.0, 30.0])
+def test_scatter_scales(device, oracle, n, decades):
+    """The temporal scatter's quotients over frames of very different noise, with
+    odd and even counts of values: mask and weighted frames equal the oracle's."""
+    rng = np.random.default_rng(n)
+    sub = rng.normal(0, 1, (n, 24, 66)) * 10.0 ** rng.uniform(-decades, decades, (n, 1, 1))
+    sub = sub.astype(np.float32)
+    sub[rng.random(sub.shape) < 0.1] = np.nan
+    t = np.linspace(-0.3, 0.3, n)
+    kw = dict(mask_scatter=1.4, weight_scatter=0.7)
+    got, want = device.stage(sub, t, 1.5, **kw), oracle.build_stage(sub, t, 1.5, **kw)
+    for k in ("sigma", "mask", "filtered"):
+        assert np.array_equal(np.asarray(got[k]), np.asarray(want[k]), equal_nan=True), k
