@@ -161,6 +161,8 @@ def _declare(L):
     L.ft_b200_result_null_peaks.argtypes = [C.c_void_p, C.c_void_p, C.c_int]
     L.ft_b200_result_maps.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
     L.ft_b200_result_velocity.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]
+    L.ft_b200_result_velocities.argtypes = [C.c_void_p, C.c_void_p, C.c_int]
+    L.ft_b200_result_track_points.argtypes = [C.c_void_p, C.c_void_p, C.c_int]
     L.ft_b200_stage.argtypes = [C.c_void_p, _f32p, C.c_int, C.c_int, C.c_int, _f64p, C.POINTER(StageParams),
                                 C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
     L.ft_b200_stage_dev.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, _f64p,
@@ -594,7 +596,10 @@ def _read_result(L, r, w, h, maps, csv_path=None):
             cnt = L.ft_b200_result_peaks(r, which, None, 0)
             arr = (Peak * max(cnt, 1))()
             L.ft_b200_result_peaks(r, which, arr, cnt)
-            return [(q.x, q.y, q.snr, q.vidx) for q in arr[:cnt]]
+            # (one conversion for all: a search may report tens of thousands)
+            fields = np.frombuffer(arr, np.dtype([("x", np.int32), ("y", np.int32), ("snr", np.float32), ("vidx", np.int32)]),
+                                   cnt)
+            return fields.tolist()
         cnt = L.ft_b200_result_null_peaks(r, None, 0)
         nulls = np.empty(cnt)
         L.ft_b200_result_null_peaks(r, nulls.ctypes.data_as(C.c_void_p), cnt)
@@ -604,27 +609,19 @@ def _read_result(L, r, w, h, maps, csv_path=None):
             bv = np.empty((h, w), np.int32)
             if L.ft_b200_result_maps(r, ms.ctypes.data_as(C.c_void_p), bv.ctypes.data_as(C.c_void_p)) != FT_B200_OK:
                 ms = bv = None  # a null-run shard other than 0 has no maps
-        grid = np.empty((nv.value, 2))
-        vx, vy = C.c_double(), C.c_double()
-        for j in range(nv.value):
-            L.ft_b200_result_velocity(r, j, C.byref(vx), C.byref(vy))
-            grid[j] = (vx.value, vy.value)
+        grid = np.zeros((nv.value, 2))
+        L.ft_b200_result_velocities(r, grid.ctypes.data_as(C.c_void_p), nv.value)
         nc = L.ft_b200_result_candidates(r, None, None, 0)
         rows = np.empty((max(nc, 1), 17))
         fl = C.create_string_buffer(64 * max(nc, 1))
         L.ft_b200_result_candidates(r, rows.ctypes.data_as(C.c_void_p), fl, nc)
-        cands = [(rows[q].copy(), fl.raw[64 * q:64 * q + 64].split(b"\0", 1)[0].decode()) for q in range(nc)]
+        flags = fl.raw
+        cands = [(rows[q].copy(), flags[64 * q:64 * q + 64].split(b"\0", 1)[0].decode()) for q in range(nc)]
         reg = DriftCheck()
         L.ft_b200_result_registration(r, C.byref(reg))
-        pt = [C.c_double() for _ in range(5)]
-        tracks = []
-        for q in range(nc):  # every frame of every candidate (ft_get_track_point)
-            f, rows_q = 0, []
-            while L.ft_b200_result_track_point(r, q, f, *[C.byref(v) for v in pt]) == FT_B200_OK:
-                rows_q.append([v.value for v in pt])
-                f += 1
-            tracks.append(rows_q)
-        track_points = np.array(tracks, np.float64).reshape(nc, -1, 5) if nc else np.zeros((0, 0, 5))
+        # every frame of every candidate (ft_get_track_point)
+        track_points = np.zeros((nc, L.ft_b200_result_track_points(r, None, 0) if nc else 0, 5))
+        L.ft_b200_result_track_points(r, track_points.ctypes.data_as(C.c_void_p), nc)
         size = L.ft_b200_result_candidates_csv(r, None, 0)
         text = C.create_string_buffer(size + 1)
         L.ft_b200_result_candidates_csv(r, text, size + 1)

@@ -880,6 +880,28 @@ int ft_b200_result_velocity(const ft_b200_result* r, int vidx, double* vx_pxh, d
     return FT_B200_OK;
 }
 
+int ft_b200_result_velocities(const ft_b200_result* r, double* v, int cap) {
+    if (!r) return 0;
+    const int count = static_cast<int>(r->o.grid.size());
+    for (int k = 0; v && k < std::min(cap, count); ++k) {
+        v[2 * k] = r->o.grid[static_cast<size_t>(k)].first;
+        v[2 * k + 1] = r->o.grid[static_cast<size_t>(k)].second;
+    }
+    return count;
+}
+
+int ft_b200_result_track_points(const ft_b200_result* r, double* points, int cap) {
+    if (!r) return 0;
+    const int frames = static_cast<int>(r->o.t_h.size());
+    const int count = std::min(cap, static_cast<int>(r->o.candidates.size()));
+    for (int c = 0; points && c < count; ++c)
+        for (int f = 0; f < frames; ++f) {
+            double* p = points + (static_cast<size_t>(c) * frames + static_cast<size_t>(f)) * 5;
+            ft_b200_result_track_point(r, c, f, p, p + 1, p + 2, p + 3, p + 4);
+        }
+    return frames;
+}
+
 int ft_b200_timings(const ft_b200_ctx* ctx, char* names, int names_len, double* seconds, int cap) {
     if (!ctx || !ctx->c) return 0;
     const auto& t = ctx->c->timings;

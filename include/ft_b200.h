@@ -369,6 +369,10 @@ int ft_b200_result_candidate(const ft_b200_result* r, int index, ft_b200_candida
  * ra_deg and dec_deg 0 (no WCS). Any output may be NULL. */
 int ft_b200_result_track_point(const ft_b200_result* r, int index, int frame, double* mjd, double* x, double* y,
                                double* ra_deg, double* dec_deg);
+/* The same of every frame of every candidate in one call: points[(c * frames + f) * 5
+ * + 0 .. 4] (mjd, x, y, ra_deg, dec_deg) for the first cap candidates; returns the
+ * frames. */
+int ft_b200_result_track_points(const ft_b200_result* r, double* points, int cap);
 /* The candidate file of the search (write_candidates_csv, io.cpp:82-115), byte
  * for byte as the reference writes it for frames without a WCS, photometric
  * calibration or near-Earth distances: two comment lines (reference epoch,
@@ -383,6 +387,9 @@ long long ft_b200_result_candidates_csv(const ft_b200_result* r, char* buf, long
 int ft_b200_result_maps(const ft_b200_result* r, float* max_snr, int* best_v);
 /* The trial motion vidx of the grid (velocity_grid, search.cpp:39-58), px/hour. */
 int ft_b200_result_velocity(const ft_b200_result* r, int vidx, double* vx_pxh, double* vy_pxh);
+/* The first cap motions of the grid in one call, v[2 k] and v[2 k + 1] of motion k;
+ * returns the count of all. */
+int ft_b200_result_velocities(const ft_b200_result* r, double* v, int cap);
 
 /* The registration check of a frame sequence (DriftCheck, registration.hpp:22-30;
  * check_registration, registration.cpp:260-312): stars (bright, extended local
