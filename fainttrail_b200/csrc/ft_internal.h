@@ -139,6 +139,7 @@ void allow_dynamic_smem(const void* func, size_t bytes);
 // 7 = 32 x 12 (16 warps), 8 = 32 x 20 with the shared maximum (16 warps).
 constexpr int kStackShapes = 8;
 constexpr int kStreamShape = 6;
+constexpr int kPairShape = 9;  // 32 x 12, 8 warps, two CTAs an SM: only by the automatic choice
 StackConfig stack_shape_config(int shape, int device_smem_optin);
 bool stack_shape_fits(const StackConfig& c, int n);
 // A process-wide choice for choose_stack_config: 0 = by frame count, else a shape

@@ -245,6 +245,10 @@ StackConfig stack_shape_config(int shape, int smem_optin) {
             c.tile_w = 32; c.wp = 40; c.p = 20; c.ty = 16; c.merge = 1; c.rows = shape_row_spread(20, 1);
             c.smem_bytes -= 32 * 20 * 8;
             break;
+        case kPairShape:
+            c.tile_w = 32; c.wp = 40; c.p = 12; c.ty = 8; c.rows = shape_row_spread(12, 0);
+            c.smem_bytes = std::min(smem_optin - 1024, 111 * 1024);  // two CTAs an SM
+            break;
         default: throw std::runtime_error("stack: unknown tile shape");
     }
     return c;
@@ -274,16 +278,18 @@ constexpr long long kStreamPixelsAhead = 200000;
 
 }  // namespace
 
-// Whether most blocks keep to row offsets of 1, as the 32 x 12 and the
-// shared-maximum kernels take them (others are cut, and their rests padded): a
-// sample of blocks, every frame.
-static bool close_rows(int n, const int* dx, const int* dy, const std::vector<int>& order) {
+// What most blocks are, by a sample of them over every frame: kClose with one column
+// and row offsets of at most 1, as the 32 x 12 and the shared-maximum kernels'
+// row-descriptor path takes them (others with one column are cut, and their rests
+// padded); kApart without a shared column.
+enum Blocks { kClose, kApart, kWide };
+static Blocks block_kind(int n, const int* dx, const int* dy, const std::vector<int>& order) {
     constexpr size_t M = kMotionBlock;
     const size_t nblk = order.size() / M, step = std::max<size_t>(1, nblk / 64);
-    size_t seen = 0, wide = 0;
+    size_t seen = 0, wide = 0, apart = 0;
     for (size_t b = 0; b < nblk; b += step, ++seen) {
-        bool far = false;
-        for (int i = 0; i < n && !far; ++i) {
+        bool rows = false, columns = false;
+        for (int i = 0; i < n && !columns; ++i) {
             int lx = INT32_MAX, hx = INT32_MIN, ly = INT32_MAX, hy = INT32_MIN;
             for (size_t k = 0; k < M; ++k) {
                 const int j = order[b * M + k];
@@ -294,11 +300,13 @@ static bool close_rows(int n, const int* dx, const int* dy, const std::vector<in
                 ly = std::min(ly, dy[e]);
                 hy = std::max(hy, dy[e]);
             }
-            far = lx < hx || static_cast<long long>(hy) - ly > 1;
+            columns = lx < hx;
+            rows = rows || static_cast<long long>(hy) - ly > 1;
         }
-        wide += far;
+        apart += columns;
+        wide += rows || columns;
     }
-    return wide * 10 <= seen;
+    return wide * 10 <= seen ? kClose : apart * 2 > seen ? kApart : kWide;
 }
 
 StackConfig choose_stack_config(int n, const int* dx, const int* dy, const std::vector<int>& order, int smem_optin) {
@@ -313,11 +321,14 @@ StackConfig choose_stack_config(int n, const int* dx, const int* dy, const std::
     // per-thread maxima 78.3; 12 frames of 1024 x 768 1.74 against 1.82 ms); then
     // 32 x 16 with the shared maximum (33 frames of 2048^2 24.3 ms, 32 x 12 24.5,
     // per-thread 25.6; 10 passes of 30 frames of 1024^2 268, 273 and 283 ms); then
-    // 32 x 12 to 62 frames (56 frames of 2048 x 1024 50.2 ms, 32 x 8 79.7). Other
-    // motions: 32 x 16 with per-thread maxima. Taller frame stacks need the shorter
-    // tiles.
-    const bool close = close_rows(n, dx, dy, order);
-    for (int s : {close ? (n <= kShortRows ? 7 : 5) : 1, close ? 7 : 3, 3}) {
+    // 32 x 12 to 62 frames (56 frames of 2048 x 1024 50.2 ms, 32 x 8 79.7). Motions
+    // without shared columns, whose groups are small: to 31 frames two CTAs of 32 x 12
+    // an SM, one of which adds while the other's windows arrive (30 frames of 1000 x
+    // 700, 4912 curved motions 15.3 ms, 32 x 16 alone on its SM 18.2; 16 of 2000 x 1400
+    // 13.3 and 14.1). Else 32 x 16 with per-thread maxima; taller frame stacks need the
+    // shorter tiles.
+    const Blocks kind = block_kind(n, dx, dy, order);
+    for (int s : {kind == kClose ? (n <= kShortRows ? 7 : 5) : kind == kApart ? kPairShape : 1, kind == kClose ? 7 : 1, 3}) {
         const StackConfig c = stack_shape_config(s, smem_optin);
         if (stack_shape_fits(c, n)) return c;
     }
@@ -385,7 +396,7 @@ StackPlan make_stack_plan(int w, int h, int n, const int* dx, const int* dy, int
     for (size_t b = 0; b < order.size(); b += M) {
         long long rows = 0;
         int real = 0;
-        bool fits = true;
+        bool fits = true, column = true;  // column: shared in every frame
         for (int k = 0; k < M; ++k) real += order[b + k] >= 0;
         for (int i = 0; i < n && real > 1; ++i) {
             int lx = INT32_MAX, hx = INT32_MIN, ly = INT32_MAX, hy = INT32_MIN;
@@ -397,6 +408,7 @@ StackPlan make_stack_plan(int w, int h, int n, const int* dx, const int* dy, int
                 ly = std::min(ly, cdy(j, i));
                 hy = std::max(hy, cdy(j, i));
             }
+            column = column && lx == hx;
             if (hx - floor4(lx) + TW > WP) fits = false;
             rows += roundup(TH + hy - ly, BH);
         }
@@ -405,9 +417,9 @@ StackPlan make_stack_plan(int w, int h, int n, const int* dx, const int* dy, int
         if (real > 1 && (!fits || rows * WP + table1 > budget)) {
             for (int k = 0; k < M; ++k)
                 if (order[b + k] >= 0) blocks.insert(blocks.end(), {order[b + k], -1, -1, -1});
-        } else if (real > 1 && cfg.rows > 0 && cfg.rows < kRowSpread) {
-            // a kernel that takes smaller row offsets: consecutive runs of the
-            // block whose rows stay within cfg.rows in every frame
+        } else if (real > 1 && column && cfg.rows > 0 && cfg.rows < kRowSpread) {
+            // a kernel that takes smaller row offsets in its row-descriptor path:
+            // consecutive runs of the block whose rows stay within cfg.rows in every frame
             std::vector<int> run;
             std::vector<int> lo(static_cast<size_t>(n)), hi(static_cast<size_t>(n));
             auto close = [&]() {
@@ -1591,7 +1603,7 @@ __device__ bool stack_tile2(const StackArgs& a, const CUtensorMap* tmap, int x0,
 // the SMs stay busy to the end. TW: tile width, 32 (one column per thread) or
 // 64 (paired columns).
 template <int NW, int P, int WP, int BH, int TW, int MERGE>
-__global__ void __launch_bounds__(32 * NW, 1)
+__global__ void __launch_bounds__(32 * NW, NW <= 8 ? 2 : 1)
     stack_batch_kernel(const StackArgs* __restrict__ passes, const CUtensorMap* __restrict__ maps, int npasses,
                        long long items, int* queue, int* err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1696,7 +1708,7 @@ void launch_batch(const std::vector<BatchPass>& batch, unsigned char* d_desc, si
     FTB_CHECK(cudaMemcpyAsync(d_desc, host.data(), host.size(), cudaMemcpyHostToDevice, s));
     auto kern = stack_batch_kernel<NW, P, WP, BH, TW, MERGE>;
     allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
-    const int ctas = static_cast<int>(std::min<long long>(items, sms));
+    const int ctas = static_cast<int>(std::min<long long>(items, NW <= 8 ? 2 * sms : sms));
     kern<<<ctas, 32 * NW, smem, s>>>(reinterpret_cast<const StackArgs*>(d_desc + 128 + 128 * np),
                                      reinterpret_cast<const CUtensorMap*>(d_desc + 128), static_cast<int>(np), items,
                                      reinterpret_cast<int*>(d_desc), d_err);
@@ -1728,7 +1740,8 @@ void stack_launch_batch(const std::vector<BatchPass>& batch, unsigned char* d_de
         launch_batch<16, 12, 40, 4, 32, 0>(batch, d_desc, desc_bytes, d_err, sms, s);
     else if (c.tile_w == 32 && c.wp == 40 && c.ty == 16 && c.p == 20 && c.merge == 1)
         launch_batch<16, 20, 40, 4, 32, 1>(batch, d_desc, desc_bytes, d_err, sms, s);
-
+    else if (c.tile_w == 32 && c.wp == 40 && c.ty == 8 && c.p == 12 && c.merge == 0)
+        launch_batch<8, 12, 40, 4, 32, 0>(batch, d_desc, desc_bytes, d_err, sms, s);
     else
         throw std::runtime_error("stack: unsupported tile shape");
 }
