@@ -45,6 +45,7 @@ struct SkyArgs {
     const unsigned char* rank;         // time rank of each frame
     const unsigned char* frame_of;     // frame of each time rank
     int w, h, pitch, n, exclude, need;
+    int sub_pitch;  // of sub, any
 };
 
 // One thread per pixel. The pixel's values are held in time-rank order, so the
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(64) sky_kernel(const SkyArgs a) {
     const size_t pix = static_cast<size_t>(y) * a.pitch + x;
     int m_all = 0;
     for (int r = 0; r < n; ++r) {
-        const float v = a.sub[a.frame_of[r] * plane + pix];
+        const float v = a.sub[a.frame_of[r] * (static_cast<size_t>(a.sub_pitch) * a.h) + static_cast<size_t>(y) * a.sub_pitch + x];
         const bool fin = finitef(v);
         V[r * T + t] = fin ? v : CUDART_INF_F;
         m_all += fin;
@@ -305,23 +306,27 @@ __global__ void __launch_bounds__(sky_threads(N)) sky_middle_kernel(const SkyArg
     constexpr int kSure = sizeof(Mask) > 4 ? 0 : N <= 64 ? N - 8 : N - 16;
     constexpr bool kHeld = N <= 64;  // the values stay in shared memory; more are read again
     const int t = threadIdx.x, n = a.n, e = min(a.exclude, n), most = sky_middle(n, e), rows = sky_rows(most);
-    size_t* at = reinterpret_cast<size_t*>(sm);       // [n] a rank's frame, from the first pixel
-    float* S = reinterpret_cast<float*>(at + n) + t;  // [rows][T] the middle values, then +inf
+    size_t* at = reinterpret_cast<size_t*>(sm);           // [n] a rank's frame in the residuals, from the first pixel
+    size_t* from = at + n;                                // [n] and in sub
+    float* S = reinterpret_cast<float*>(from + n) + t;    // [rows][T] the middle values, then +inf
     float* V = S + rows * T;                          // [n][T] values by time rank, +inf if not finite
     // [n + 2 e + 1][T] by time rank, from rank -e - 1 on: none outside the sequence
     Code* code = reinterpret_cast<Code*>(S - t + T * (rows + (kHeld ? n : 0))) + t + T * (e + 1);
     const size_t plane = static_cast<size_t>(a.pitch) * a.h;
-    for (int r = t; r < n; r += T) at[r] = a.frame_of[r] * plane;
+    for (int r = t; r < n; r += T) {
+        at[r] = a.frame_of[r] * plane;
+        from[r] = a.frame_of[r] * (static_cast<size_t>(a.sub_pitch) * a.h);
+    }
     __syncthreads();
     const unsigned q = blockIdx.x * static_cast<unsigned>(T) + t;
     const int y = static_cast<int>(q / static_cast<unsigned>(a.w)), x = static_cast<int>(q - y * static_cast<unsigned>(a.w));
     if (y >= a.h) return;
     const size_t pix = static_cast<size_t>(y) * a.pitch + x;
-    const float* sub = a.sub + pix;
+    const float* sub = a.sub + static_cast<size_t>(y) * a.sub_pitch + x;
     float* residual = a.residual + pix;
     float sv[N];
 #pragma unroll
-    for (int r = 0; r < N; ++r) sv[r] = r < kSure || r < n ? __ldg(sub + at[r]) : CUDART_INF_F;
+    for (int r = 0; r < N; ++r) sv[r] = r < kSure || r < n ? __ldg(sub + from[r]) : CUDART_INF_F;
     int m_all = 0;
     bool negzero = false;
 #pragma unroll
@@ -338,7 +343,7 @@ __global__ void __launch_bounds__(sky_threads(N)) sky_middle_kernel(const SkyArg
     }
     auto value = [&](int r) {
         if (kHeld) return V[r * T];
-        const float v = sub[at[r]];
+        const float v = sub[from[r]];
         return finitef(v) ? v : CUDART_INF_F;
     };
 #pragma unroll
@@ -1105,7 +1110,7 @@ __global__ void __launch_bounds__(256) filter_kernel(const FilterArgs a) {
 template <int N, class Mask>
 void launch_sky_middle(const SkyArgs& a, long long npix, cudaStream_t s) {
     constexpr int T = sky_threads(N);
-    const size_t smem = sizeof(size_t) * a.n + static_cast<size_t>(T) *
+    const size_t smem = 2 * sizeof(size_t) * a.n + static_cast<size_t>(T) *
         (4 * sky_rows(sky_middle(a.n, a.exclude)) + ((N <= 64 ? 4 : 0) + sizeof(typename SkyCode<Mask>::type)) * a.n +
          sizeof(typename SkyCode<Mask>::type) * (2 * std::min(a.exclude, a.n) + 1));
     auto kern = sky_middle_kernel<N, Mask>;
@@ -1448,33 +1453,47 @@ void launch_filter_any(const FilterArgs& a, int n, int sms, cudaStream_t s) {
 // Bound by memory: each thread scales four columns of four rows (one pixel a thread
 // with a 64-bit division for its row: 595 us for 40 frames of 2048^2, 2.3 TB/s; now
 // 193 us).
-__global__ void __launch_bounds__(256) rescale_kernel(float* g, size_t plane, int w, int h, int pitch, const double* sg) {
+//
+// to: where the scaled frames go, rows to_pitch floats apart (g itself, or a caller's
+// buffer of any alignment: the copy out of the stage's own layout, 0.42 ms for those
+// frames, is this pass's stores).
+__global__ void __launch_bounds__(256) rescale_kernel(const float* g, size_t plane, int w, int h, int pitch, const double* sg,
+                                                      float* to, int to_pitch) {
     const int f = blockIdx.z;
     const double s = sg[f];
-    if (!(s > 0.0)) return;
-    const float ig = __double2float_rn(__ddiv_rn(1.0, s));
+    const bool scale = s > 0.0;
+    if (!scale && to == g) return;
+    const float ig = scale ? __double2float_rn(__ddiv_rn(1.0, s)) : 0.0f;
+    auto times = [&](float v) { return scale ? __fmul_rn(v, ig) : v; };
+    const bool quads = to_pitch % 4 == 0 && reinterpret_cast<uintptr_t>(to) % 16 == 0;
     const int x = 4 * static_cast<int>(blockIdx.x * 64 + (threadIdx.x & 63)), y0 = static_cast<int>(blockIdx.y * 16 + (threadIdx.x >> 6));
     if (x >= w) return;
-    float* p = g + f * plane + static_cast<size_t>(y0) * pitch + x;
-    const size_t down = 4 * static_cast<size_t>(pitch);
-    if (x + 3 < w) {
-        float4 v[4];
+    const float* p = g + f * plane + static_cast<size_t>(y0) * pitch + x;
+    float* o = to + f * (static_cast<size_t>(to_pitch) * h) + static_cast<size_t>(y0) * to_pitch + x;
+    const size_t down = 4 * static_cast<size_t>(pitch), to_down = 4 * static_cast<size_t>(to_pitch);
+    float4 v[4];  // (columns beyond w: the row's padding, not stored)
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (y0 + 4 * k < h) v[k] = *reinterpret_cast<const float4*>(p + k * down);
+    for (int k = 0; k < 4; ++k)
+        if (y0 + 4 * k < h) v[k] = *reinterpret_cast<const float4*>(p + k * down);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (y0 + 4 * k < h)
-                *reinterpret_cast<float4*>(p + k * down) =
-                    make_float4(__fmul_rn(v[k].x, ig), __fmul_rn(v[k].y, ig), __fmul_rn(v[k].z, ig), __fmul_rn(v[k].w, ig));
-    } else {
-        for (int k = 0; k < 4; ++k)
-            for (int c = 0; x + c < w && y0 + 4 * k < h; ++c) p[k * down + c] = __fmul_rn(p[k * down + c], ig);
+    for (int k = 0; k < 4; ++k) {
+        if (y0 + 4 * k >= h) break;
+        const float4 r = make_float4(times(v[k].x), times(v[k].y), times(v[k].z), times(v[k].w));
+        float* q = o + k * to_down;
+        if (quads && x + 3 < w) {
+            *reinterpret_cast<float4*>(q) = r;
+        } else {
+            q[0] = r.x;
+            if (x + 1 < w) q[1] = r.y;
+            if (x + 2 < w) q[2] = r.z;
+            if (x + 3 < w) q[3] = r.w;
+        }
     }
 }
 
-inline void launch_rescale(float* g, size_t plane, int w, int h, int pitch, int n, const double* sg, cudaStream_t s) {
-    rescale_kernel<<<dim3((w + 255) / 256, (h + 15) / 16, n), 256, 0, s>>>(g, plane, w, h, pitch, sg);
+inline void launch_rescale(const float* g, size_t plane, int w, int h, int pitch, int n, const double* sg, float* to,
+                           int to_pitch, cudaStream_t s) {
+    rescale_kernel<<<dim3((w + 255) / 256, (h + 15) / 16, n), 256, 0, s>>>(g, plane, w, h, pitch, sg, to, to_pitch);
     FTB_CHECK(cudaGetLastError());
 }
 
@@ -1630,7 +1649,7 @@ static StageTables stage_tables(StageScratch& sc, int n) {
 }
 
 void stage_noise(Context& c, StageScratch& sc, const float* d_sub, int w, int h, int n, const double* t_h,
-                 int static_exclude, float* d_sky) {
+                 int static_exclude, float* d_sky, int sub_pitch) {
     if (n < 1 || n > 255) throw std::runtime_error("stage: between 1 and 255 frames are supported");
     if (w != sc.w_ || h != sc.h_ || n != sc.n_) throw std::runtime_error("stage: scratch sized for another shape");
     const int pitch = frame_pitch(w);
@@ -1654,7 +1673,7 @@ void stage_noise(Context& c, StageScratch& sc, const float* d_sub, int w, int h,
     {
         const int span = c.span_begin("static sky + residuals");
         SkyArgs a{d_sub, sc.residual.as<float>(), d_sky, tb.tab, tb.tab + n, w, h, pitch, n, exclude,
-                  std::max(5, static_cast<int>(0.6 * n))};
+                  std::max(5, static_cast<int>(0.6 * n)), sub_pitch > 0 ? sub_pitch : pitch};
         launch_sky(a, n, npix, s);
         ++c.launches;
         c.span_end(span);
@@ -1676,7 +1695,7 @@ void stage_noise(Context& c, StageScratch& sc, const float* d_sub, int w, int h,
 }
 
 void stage_filter(Context& c, StageScratch& sc, int w, int h, int n, const StageParams& sp, float* d_filtered,
-                  float* d_mask, double* h_sigma, int* h_cr) {
+                  float* d_mask, double* h_sigma, int* h_cr, float* d_out, int out_pitch) {
     if (!sc.fits(w, h, n, sp.fwhm_px)) throw std::runtime_error("stage: scratch sized for another shape");
     const int pitch = frame_pitch(w);
     const size_t plane = static_cast<size_t>(pitch) * h;
@@ -1752,7 +1771,7 @@ void stage_filter(Context& c, StageScratch& sc, int w, int h, int n, const Stage
         }
         launch_select<false>(sc.samples.as<float>(), sc.cap, d_counts, n, d_sg, 0, s);
         ++c.launches;
-        launch_rescale(d_filtered, plane, w, h, pitch, n, d_sg, s);
+        launch_rescale(d_filtered, plane, w, h, pitch, n, d_sg, d_out ? d_out : d_filtered, d_out ? out_pitch : pitch, s);
         ++c.launches;
         c.span_end(span);
     }
@@ -1761,9 +1780,10 @@ void stage_filter(Context& c, StageScratch& sc, int w, int h, int n, const Stage
 }
 
 void stage_run(Context& c, StageScratch& sc, const float* d_sub, int w, int h, int n, const double* t_h,
-               const StageParams& sp, float* d_filtered, float* d_sky, float* d_mask, double* h_sigma, int* h_cr) {
-    stage_noise(c, sc, d_sub, w, h, n, t_h, sp.static_exclude, d_sky);
-    stage_filter(c, sc, w, h, n, sp, d_filtered, d_mask, h_sigma, h_cr);
+               const StageParams& sp, float* d_filtered, float* d_sky, float* d_mask, double* h_sigma, int* h_cr,
+               int sub_pitch, float* d_out, int out_pitch) {
+    stage_noise(c, sc, d_sub, w, h, n, t_h, sp.static_exclude, d_sky, sub_pitch);
+    stage_filter(c, sc, w, h, n, sp, d_filtered, d_mask, h_sigma, h_cr, d_out, out_pitch);
 }
 
 void stage_sigma_to_host(Context& c, StageScratch& sc, int n, double* h_sigma) {
@@ -1813,7 +1833,7 @@ void stage_sky(Context& c, StageScratch& sc, const float* d_sub, int w, int rows
     FTB_CHECK(cudaMemcpyAsync(tb.tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, s));
     const int span = c.span_begin("static sky + residuals");
     SkyArgs a{d_sub, sc.residual.as<float>(), d_sky, tb.tab, tb.tab + n, w, rows, pitch, n, exclude,
-              std::max(5, static_cast<int>(0.6 * n))};
+              std::max(5, static_cast<int>(0.6 * n)), pitch};
     launch_sky(a, n, npix, s);
     ++c.launches;
     c.span_end(span);
@@ -1919,7 +1939,7 @@ void stage_filter_given(Context& c, StageScratch& sc, int w, int rows, int n, co
         c.span_end(span);
     }
     if (d_sg) {
-        launch_rescale(d_filtered, plane, w, rows, pitch, n, d_sg, s);
+        launch_rescale(d_filtered, plane, w, rows, pitch, n, d_sg, d_filtered, pitch, s);
         ++c.launches;
     }
 }

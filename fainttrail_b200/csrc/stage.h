@@ -35,17 +35,20 @@ void stage_time_ranks(const double* t_h, int n, std::vector<int>& rank);
 // in the reference (preprocess.cpp:368): static sky, residuals and per-frame
 // noise; then scatter, mask, matched filter and its normalisation.
 void stage_noise(Context& c, StageScratch& sc, const float* d_sub, int w, int h, int n, const double* t_h,
-                 int static_exclude, float* d_sky);
+                 int static_exclude, float* d_sky, int sub_pitch = 0);
 void stage_filter(Context& c, StageScratch& sc, int w, int h, int n, const StageParams& sp, float* d_filtered,
-                  float* d_mask, double* h_sigma, int* h_cr);
+                  float* d_mask, double* h_sigma, int* h_cr, float* d_out = nullptr, int out_pitch = 0);
 void stage_sigma_to_host(Context& c, StageScratch& sc, int n, double* h_sigma);
 
-// build_stage on device frames d_sub (n x h x pitch, pitch = frame_pitch(w)):
-// d_filtered (same layout), d_sky and d_mask (h x pitch); h_sigma / h_cr (host,
-// may be null) receive the per-frame noise and cosmic-ray counts after the
-// stream is synchronised by the caller.
+// build_stage on device frames d_sub (n x h x pitch, pitch = frame_pitch(w), or
+// sub_pitch > 0: any): d_filtered (n x h x pitch), d_sky and d_mask (h x pitch); h_sigma
+// / h_cr (host, may be null) receive the per-frame noise and cosmic-ray counts after
+// the stream is synchronised by the caller. With d_out the normalised frames go there
+// (n x h x out_pitch, any alignment; only after d_sub was read for the last time) and
+// d_filtered holds them unnormalised.
 void stage_run(Context& c, StageScratch& sc, const float* d_sub, int w, int h, int n, const double* t_h,
-               const StageParams& sp, float* d_filtered, float* d_sky, float* d_mask, double* h_sigma, int* h_cr);
+               const StageParams& sp, float* d_filtered, float* d_sky, float* d_mask, double* h_sigma, int* h_cr,
+               int sub_pitch = 0, float* d_out = nullptr, int out_pitch = 0);
 
 // Median and robust sigma (common.hpp:64-82) of the regular sample of each of k
 // device frames (sample_pixels(frame, 200000), common.hpp:85-100; w x h, rows
