@@ -1484,7 +1484,7 @@ __global__ void __launch_bounds__(256) rescale_kernel(const float* g, size_t pla
     const float ig = scale ? __double2float_rn(__ddiv_rn(1.0, s)) : 0.0f;
     auto times = [&](float v) { return scale ? __fmul_rn(v, ig) : v; };
     const bool quads = to_pitch % 4 == 0 && reinterpret_cast<uintptr_t>(to) % 16 == 0;
-    const int x = 4 * static_cast<int>(blockIdx.x * 64 + (threadIdx.x & 63)), y0 = static_cast<int>(blockIdx.y * 16 + (threadIdx.x >> 6));
+    const int x = 4 * static_cast<int>(blockIdx.y * 64 + (threadIdx.x & 63)), y0 = static_cast<int>(blockIdx.x * 16 + (threadIdx.x >> 6));
     if (x >= w) return;
     const float* p = g + f * plane + static_cast<size_t>(y0) * pitch + x;
     float* o = to + f * (static_cast<size_t>(to_pitch) * h) + static_cast<size_t>(y0) * to_pitch + x;
@@ -1509,9 +1509,10 @@ __global__ void __launch_bounds__(256) rescale_kernel(const float* g, size_t pla
     }
 }
 
+// (rows along the grid's x, which has no limit of 65,535)
 inline void launch_rescale(const float* g, size_t plane, int w, int h, int pitch, int n, const double* sg, float* to,
                            int to_pitch, cudaStream_t s) {
-    rescale_kernel<<<dim3((w + 255) / 256, (h + 15) / 16, n), 256, 0, s>>>(g, plane, w, h, pitch, sg, to, to_pitch);
+    rescale_kernel<<<dim3((h + 15) / 16, (w + 255) / 256, n), 256, 0, s>>>(g, plane, w, h, pitch, sg, to, to_pitch);
     FTB_CHECK(cudaGetLastError());
 }
 
@@ -1533,7 +1534,7 @@ __global__ void __launch_bounds__(256) subtract_grow_kernel(const float* __restr
     constexpr int R = kPrepRows + 2 * kGrow, K = (R + 7) / 8;
     __shared__ unsigned char bad[R][32];
     const int f = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x = static_cast<int>(blockIdx.x) * 128 + 4 * lane, y0 = static_cast<int>(blockIdx.y) * kPrepRows;
+    const int x = static_cast<int>(blockIdx.y) * 128 + 4 * lane, y0 = static_cast<int>(blockIdx.x) * kPrepRows;
     const double b = bg[f];
     const float* src = in + f * plane;
     // four columns of a row and the bits of the non-finite ones; columns outside the image are not
@@ -1589,7 +1590,7 @@ __global__ void __launch_bounds__(256) subtract_grow_kernel(const float* __restr
 
 inline void launch_subtract_grow(const float* in, float* out, size_t plane, int w, int h, int pitch, int n, const double* bg,
                                  cudaStream_t s) {
-    subtract_grow_kernel<<<dim3((w + 127) / 128, (h + kPrepRows - 1) / kPrepRows, n), 256, 0, s>>>(in, out, plane, w, h,
+    subtract_grow_kernel<<<dim3((h + kPrepRows - 1) / kPrepRows, (w + 127) / 128, n), 256, 0, s>>>(in, out, plane, w, h,
                                                                                                     pitch, bg);
     FTB_CHECK(cudaGetLastError());
 }
