@@ -4,7 +4,7 @@
 //
 //  sky_kernel      static sky + leave-out residuals (preprocess.cpp:154-204)
 //  sample + select per-frame residual noise: regular sample grid, exact medians
-//                  by radix select (common.hpp:64-100, preprocess.cpp:356-365)
+//                  by bracketing and radix selection (common.hpp:64-100, preprocess.cpp:356-365)
 //  scatter_kernel  temporal scatter (preprocess.cpp:373-391)
 //  mask_kernel     dilated scatter mask (preprocess.cpp:392-400)
 //  filter_kernel   normalise + weight, cosmic-ray rejection, clip, separable
