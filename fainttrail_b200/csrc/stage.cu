@@ -820,6 +820,8 @@ __global__ void __cluster_dims__(kSelCluster, 1, 1) __launch_bounds__(kSelThread
     const int cnt = min(counts[f], cap);
     const float* x = samples + static_cast<size_t>(f) * cap;
     double r = 0.0;
+    // every CTA of the cluster has started before any writes to another's shared memory
+    cg::this_cluster().sync();
     if (MEDIAN) {
         if (cnt > 0) r = cluster_median<0>(x, cnt, 0.0, sh);
     } else {
