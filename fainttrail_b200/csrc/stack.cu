@@ -1616,6 +1616,7 @@ __global__ void __launch_bounds__(32 * NW, NW <= 8 ? 2 : 1)
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(base + 128);
     float* win = reinterpret_cast<float*>(base + 128 + (MERGE ? 32 * P * 8 : 0));
     if (threadIdx.x == 0) mbar_init(bar, 1);
+    tensor_maps_acquire(maps, npasses);
     __syncthreads();
     uint32_t phase = 0;
     for (;;) {

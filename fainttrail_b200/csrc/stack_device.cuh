@@ -48,6 +48,16 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
+// The tensor maps of a launch lie in global memory, at an address that earlier launches
+// used for other maps: a copy from the host wrote them, and the loads read them through
+// the tensor-map proxy. One fence a map, by the CTA's threads in turn, orders the two; the
+// CTA's barrier has to follow before the first load.
+__device__ __forceinline__ void tensor_maps_acquire(const CUtensorMap* maps, int count) {
+    for (int k = static_cast<int>(threadIdx.x); k < count; k += static_cast<int>(blockDim.x))
+        asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(maps + k))
+                     : "memory");
+}
+
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Bounded wait on the staging barrier: `limit` clock cycles (about two seconds

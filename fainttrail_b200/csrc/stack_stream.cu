@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         sh.next.g = sh.next.gb = 0;
     }
     for (int q = tid; q < 32 * P; q += kThreads) sh.keys[q] = 0ull;
+    tensor_maps_acquire(maps, npasses);
     __syncthreads();
     if (warp == 0)
         for (int b = 0; b < kBuffers; ++b)
