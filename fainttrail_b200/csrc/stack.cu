@@ -775,16 +775,36 @@ __device__ __forceinline__ void merge_max(float b, int bj, float& best, int& arg
     }
 }
 
+// Frames counted for each of a column's P pixel rows: a byte a row, and 16 bits a row for
+// tiles of four rows, the only ones whose windows of more than 255 frames fit in shared
+// memory (launch_batch checks it).
+template <int P>
+struct RowCounts {
+    static constexpr int bits = P <= 4 ? 16 : 8, per = 32 / bits, words = (P + per - 1) / per;
+    uint32_t c[words] = {};
+    // one frame more for the rows whose bit is set
+    __device__ __forceinline__ void add(uint32_t rows) {
+#pragma unroll
+        for (int w = 0; w < words; ++w) {
+            const uint32_t m = rows >> (per * w);
+            c[w] += bits == 8 ? ((m & 15u) * 0x00204081u) & 0x01010101u : (m & 1u) | (m & 2u) << 15;
+        }
+    }
+    __device__ __forceinline__ int at(int p) const {
+        return static_cast<int>((c[p / per] >> (bits * (p % per))) & (bits == 8 ? 0xffu : 0xffffu));
+    }
+};
+
 // The frames that cover this thread's P pixels (one column) for a motion, counted
 // after its sums: each lane looks at a frame's shift, the frames that cover the whole
 // tile (the common case) are a population count, those whose rows all lie inside add
-// to this column alone, and the others one byte a row (255 frames at most). Counted
-// between the adds, frame by frame and pixel by pixel, 30 frames of 1000 x 700 with
-// 4912 curved motions took 21.4 ms, now 18.2.
+// to this column alone, and the others are counted by row. Counted between the adds,
+// frame by frame and pixel by pixel, 30 frames of 1000 x 700 with 4912 curved motions
+// took 21.4 ms, now 18.2.
 template <int P>
 struct SlotCoverage {
     int column = 0;
-    uint32_t part[(P + 3) / 4] = {};
+    RowCounts<P> part;
     __device__ __forceinline__ void count(const StackArgs& a, const short2* shift, int x, int x0, int y0) {
         const int n = a.n, lane = x - x0;
         for (int c = 0; c < n; c += 32) {
@@ -799,19 +819,14 @@ struct SlotCoverage {
                 const int fx = __shfl_sync(0xffffffffu, sh.x, f), fy = __shfl_sync(0xffffffffu, sh.y, f);
                 const bool inx = static_cast<unsigned>(x + fx) < static_cast<unsigned>(a.w);
                 const int lo = max(0, -(y0 + fy)), hi = min(P - 1, a.h - 1 - (y0 + fy));
-                if (lo == 0 && hi == P - 1) {
+                if (lo == 0 && hi == P - 1)
                     column += inx;
-                } else if (lo <= hi) {
-                    const uint32_t m = inx ? (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo) : 0u;
-#pragma unroll
-                    for (int w = 0; w < (P + 3) / 4; ++w) part[w] += (((m >> (4 * w)) & 15u) * 0x00204081u) & 0x01010101u;
-                }
+                else if (lo <= hi)
+                    part.add(inx ? (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo) : 0u);
             }
         }
     }
-    __device__ __forceinline__ int frames(int p) const {
-        return column + static_cast<int>((part[p >> 2] >> (8 * (p & 3))) & 0xffu);
-    }
+    __device__ __forceinline__ int frames(int p) const { return column + part.at(p); }
 };
 
 // One block of 4 consecutive motions of a group for this thread's P pixels
@@ -906,17 +921,13 @@ __device__ __forceinline__ void add_pattern(float2 (&acc)[4][H], const float2* A
 
 // Coverage of a border tile's pixels by a block's motions: cx counts the frames
 // whose rows cover the whole tile for every motion and whose column covers
-// this thread's pixels; cpart[k] holds, one byte a row, the frames that cover
-// row p of motion k's pixels otherwise. A pixel's frame count is cx plus its
-// byte (frames never exceed 255).
+// this thread's pixels; part[k] counts by row the frames that cover motion k's
+// pixels otherwise. A pixel's frame count is their sum.
 template <int P>
 struct BorderCount {
-    static constexpr int PW = (P + 3) / 4;
     int cx = 0;
-    uint32_t cpart[4][PW] = {};
-    __device__ __forceinline__ int count(int k, int p) const {
-        return cx + static_cast<int>((cpart[k][p >> 2] >> (8 * (p & 3))) & 0xffu);
-    }
+    RowCounts<P> part[4];
+    __device__ __forceinline__ int count(int k, int p) const { return cx + part[k].at(p); }
 };
 
 // One block of 4 motions of a rows_fast group for this thread's P pixels (one
@@ -969,11 +980,7 @@ __device__ __forceinline__ void rows_accumulate(const StackArgs& a, const StackG
                     const int dy = dylow + static_cast<int>((d >> (16 + 2 * k)) & 3u);
                     const int lo = max(0, -(y0 + dy)), hi = min(P - 1, a.h - 1 - (y0 + dy));
                     if (lo > hi) continue;
-                    // rows lo..hi as bits, then each row's bit as one byte of its word
-                    const uint32_t m = (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo);
-#pragma unroll
-                    for (int w = 0; w < BorderCount<P>::PW; ++w)
-                        cov.cpart[k][w] += (((m >> (4 * w)) & 15u) * 0x00204081u) & 0x01010101u;
+                    cov.part[k].add((0xffffffffu >> (31 - hi)) & (0xffffffffu << lo));  // rows lo..hi
                 }
             }
         }
@@ -1658,6 +1665,7 @@ void launch_batch(const std::vector<BatchPass>& batch, unsigned char* d_desc, si
         const StackPlan& plan = *bp.plan;
         if (plan.cfg.ty != NW || plan.cfg.p != P || plan.cfg.tile_w != TW || plan.cfg.wp != WP || plan.cfg.merge != MERGE)
             throw std::runtime_error("stack batch: passes of different kernel shapes");
+        if (plan.n > 255 && P > 4) throw std::runtime_error("stack batch: more than 255 frames on tall tiles");
         const cuuint64_t dims[3] = {static_cast<cuuint64_t>(plan.w), static_cast<cuuint64_t>(plan.h),
                                     static_cast<cuuint64_t>(plan.n)};
         const cuuint64_t strides[2] = {static_cast<cuuint64_t>(plan.pitch) * 4,
