@@ -898,11 +898,9 @@ __device__ __forceinline__ void motion_quad(const StackArgs& a, const StackGroup
 
 // ---- one shared maximum per tile: instead of a best/argmax pair per pixel in
 // every thread, the CTA's warps merge into one array of 64-bit keys in shared
-// memory with atomicMax. key = (order-preserving bits of S/N) << 32 | ~index,
-// so a larger S/N wins and equal S/N goes to the lower motion index -- the
-// reference's rule. S/N is never -0.0 (sums start at +0.0f and round to
-// nearest) and -inf / NaN never enter, as in the register rule. Frees 2P
-// registers per thread, so 16-row tiles run 16 warps.
+// memory with atomicMax. The keys (snr_key) order by S/N, of equal S/N the lower
+// motion index first -- the reference's rule -- and -inf / NaN never enter, as in
+// the register rule. Frees 2P registers per thread, so 16-row tiles run 16 warps.
 
 // Pairs of floats: __fadd2_rn / __fmul2_rn are two independent
 // round-to-nearest operations per call, bit-identical to two scalar ones

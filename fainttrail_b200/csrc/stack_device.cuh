@@ -81,19 +81,20 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
         : "memory");
 }
 
-// A tile's shared maximum: key = (order-preserving bits of S/N) << 32 | ~index,
-// so a larger S/N wins and equal S/N goes to the lower motion index (the two zeros
-// are equal: + 0.0f makes both +0).
+// A tile's shared maximum: key = (order-preserving bits of S/N) << 32 | (~index) << 1 |
+// sign, so a larger S/N wins and equal S/N goes to the lower motion index. The two zeros
+// are equal (+ 0.0f gives both the bits of +0); the winner's own sign is in the lowest bit.
 __device__ __forceinline__ unsigned long long snr_key(float s, int j) {
     const uint32_t b = __float_as_uint(__fadd_rn(s, 0.0f));
     const uint32_t o = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-    return (static_cast<unsigned long long>(o) << 32) | static_cast<uint32_t>(~j);
+    return (static_cast<unsigned long long>(o) << 32) |
+           __funnelshift_l(__float_as_uint(s), ~static_cast<uint32_t>(j), 1);
 }
 
 __device__ __forceinline__ void snr_unkey(unsigned long long k, float& s, int& j) {
-    const uint32_t o = static_cast<uint32_t>(k >> 32);
-    s = __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-    j = static_cast<int>(~static_cast<uint32_t>(k));
+    const uint32_t o = static_cast<uint32_t>(k >> 32), low = static_cast<uint32_t>(k);
+    s = __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) | low << 31 : ~o);
+    j = static_cast<int>(low >> 1 ^ 0x7fffffffu);
 }
 
 }  // namespace ftb
