@@ -7,6 +7,7 @@
 #include <chrono>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <thread>
 #include <tuple>
 #include <cmath>
@@ -561,6 +562,33 @@ StackPlan plan_job(int smem_optin, const PassJob& j) {
     return plan;
 }
 
+// make(k) of every k, on up to 16 host threads; their time counts as "plans".
+template <class Make>
+void plan_together(Context& c, const std::vector<size_t>& todo, Make make) {
+    if (todo.empty()) return;
+    const double t0 = wall_seconds();
+    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    const size_t workers = std::min<size_t>(hw, todo.size());
+    std::vector<std::exception_ptr> errs(workers);
+    auto work = [&](size_t wkr) {
+        try {
+            for (size_t q = wkr; q < todo.size(); q += workers) make(todo[q]);
+        } catch (...) {
+            errs[wkr] = std::current_exception();
+        }
+    };
+    if (workers == 1) {
+        work(0);
+    } else {
+        std::vector<std::thread> pool;
+        for (size_t wkr = 0; wkr < workers; ++wkr) pool.emplace_back(work, wkr);
+        for (auto& t : pool) t.join();
+    }
+    for (auto& e : errs)
+        if (e) std::rethrow_exception(e);
+    c.host_time("plans", wall_seconds() - t0);
+}
+
 }  // namespace
 
 PlanAhead plan_ahead(Context& c, std::vector<PassJob> tables) {
@@ -605,40 +633,24 @@ void stack_passes_device(Context& c, std::vector<PassJob>& jobs, PlanAhead* ahea
         FTB_CHECK(cudaStreamSynchronize(c.stream()));
         return;
     }
-    const double t0 = wall_seconds();
     // plans made ahead, or on host threads now (the GPU keeps running whatever
     // was queued before)
     std::vector<StackPlan> plans(jobs.size());
     const bool use = ahead && ahead->shape == stack_shape();
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    const size_t workers = std::min<size_t>(hw, jobs.size());
-    std::vector<std::thread> pool;
-    std::vector<std::exception_ptr> errs(workers);
-    auto work = [&](size_t wkr) {
-        try {
-            for (size_t k = wkr; k < jobs.size(); k += workers) {
-                if (use && k < ahead->plans.size() && ahead->plans[k].valid()) {
-                    plans[k] = ahead->plans[k].get();  // the tables are the job's
-                    plans[k].pitch = jobs[k].pitch;
-                } else {
-                    plans[k] = plan_job(c.smem_optin(), jobs[k]);
-                }
-            }
-        } catch (...) {
-            errs[wkr] = std::current_exception();
-        }
-    };
-    if (workers == 1) {
-        work(0);
-    } else {
-        for (size_t wkr = 0; wkr < workers; ++wkr) pool.emplace_back(work, wkr);
-        for (auto& t : pool) t.join();
-    }
-    for (auto& e : errs)
-        if (e) std::rethrow_exception(e);
-    c.host_time("plans", wall_seconds() - t0);
-    // the passes left to the autotuner (its probes run on the stream, before
-    // this batch's launches); a streamed pass of that size is noted beside them
+    std::vector<size_t> todo(jobs.size());
+    std::iota(todo.begin(), todo.end(), size_t{0});
+    plan_together(c, todo, [&](size_t k) {
+        if (use && k < ahead->plans.size() && ahead->plans[k].valid())
+            plans[k] = ahead->plans[k].get();  // the tables are the job's
+        else
+            plans[k] = plan_job(c.smem_optin(), jobs[k]);
+        plans[k].pitch = jobs[k].pitch;
+    });
+    // the passes left to the autotuner: all their shapes first (its probes run on
+    // the stream, before this batch's launches), then their plans together; a
+    // streamed pass of that size is noted beside them
+    todo.clear();
+    std::vector<int> shape_of(jobs.size(), 0);
     for (size_t k = 0; k < jobs.size(); ++k) {
         const PassJob& j = jobs[k];
         if (!plans[k].stream.empty()) {
@@ -646,12 +658,15 @@ void stack_passes_device(Context& c, std::vector<PassJob>& jobs, PlanAhead* ahea
                 std::lock_guard<std::mutex> lk(g_tune_mu);
                 g_tuned.emplace(std::make_tuple(j.n, j.m, j.w, j.h), kStreamShape);
             }
-            continue;
+        } else if (plans[k].m == 0) {
+            shape_of[k] = autotune_shape(c, j);
+            todo.push_back(k);
         }
-        if (plans[k].m > 0) continue;
-        plans[k] = resident_plan(c.smem_optin(), j, autotune_shape(c, j));
-        plans[k].pitch = j.pitch;
     }
+    plan_together(c, todo, [&](size_t k) {
+        plans[k] = resident_plan(c.smem_optin(), jobs[k], shape_of[k]);
+        plans[k].pitch = jobs[k].pitch;
+    });
     // the streamed passes, small ones cut into several work items a tile, whose
     // maxima then merge in global keys (without room for those: one item a tile)
     std::vector<size_t> streamed;
