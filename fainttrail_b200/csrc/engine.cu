@@ -1,6 +1,7 @@
 // Device context and the stacking-pass driver of the B200 backend.
 #include "engine.h"
 
+#include "caller_memory.h"
 #include "stage.h"
 
 #include <algorithm>
@@ -362,37 +363,47 @@ void stack_pass_host(Context& c, const float* frames, int w, int h, int n, const
 
 namespace {
 
+bool in_place(const Context& c, const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return ftb::in_place(a, c.device());
+    cudaGetLastError();
+    return false;  // the copies say what is wrong with it
+}
+
 // build_stage with the caller's frames and outputs in host memory (io_pitch =
-// w), copied to and from the stage's own layout around the device stage, or device
-// memory (rows io_pitch floats apart): the sky kernel then reads the caller's frames
-// and the normalisation writes the caller's, which may be the same.
+// w) or device memory (rows io_pitch floats apart), copied to and from the stage's
+// own layout around the device stage. Of this GPU's memory nothing is copied: the sky
+// kernel reads the caller's frames and the normalisation writes the caller's, which
+// may be the same.
 void stage_io(Context& c, const float* sub, bool on_device, int io_pitch, int w, int h, int n, const double* t_h,
               const StageParams& sp, float* filtered, float* static_sky, float* mask, double* sigma, int* cr) {
     c.bind();
     const int pitch = frame_pitch(w);
     const size_t plane = static_cast<size_t>(pitch) * h;
+    const cudaMemcpyKind in_kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     const cudaMemcpyKind out_kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     const size_t io_row = sizeof(float) * static_cast<size_t>(io_pitch);
+    const bool read_there = on_device && in_place(c, sub), write_there = on_device && filtered && in_place(c, filtered);
     c.timing_reset();
     const float* d_sub = sub;
-    float* d_frames = on_device ? nullptr : c.scratch(kFrames, sizeof(float) * plane * n, "frames").as<float>();
+    float* d_frames = read_there ? nullptr : c.scratch(kFrames, sizeof(float) * plane * n, "frames").as<float>();
     float* d_filt = c.scratch(kStageOut, sizeof(float) * plane * n, "filtered frames").as<float>();
     float* d_sky = c.scratch(kSky, sizeof(float) * plane, "static sky").as<float>();
     float* d_mask = c.scratch(kMask, sizeof(float) * plane, "mask").as<float>();
     StageScratch sc(c, w, h, n, sp.fwhm_px);
     const int up = c.span_begin("upload");
-    if (!on_device) {
+    if (!read_there) {
         FTB_CHECK(cudaMemcpy2DAsync(d_frames, sizeof(float) * pitch, sub, io_row, sizeof(float) * w,
-                                    static_cast<size_t>(h) * n, cudaMemcpyHostToDevice, c.stream()));
+                                    static_cast<size_t>(h) * n, in_kind, c.stream()));
         d_sub = d_frames;
     }
     c.span_end(up);
     std::vector<double> sg(static_cast<size_t>(n));
     std::vector<int> crv(static_cast<size_t>(n));
-    stage_run(c, sc, d_sub, w, h, n, t_h, sp, d_filt, d_sky, d_mask, sg.data(), crv.data(), on_device ? io_pitch : pitch,
-              on_device ? filtered : nullptr, io_pitch);
+    stage_run(c, sc, d_sub, w, h, n, t_h, sp, d_filt, d_sky, d_mask, sg.data(), crv.data(), read_there ? io_pitch : pitch,
+              write_there ? filtered : nullptr, io_pitch);
     const int down = c.span_begin("download");
-    if (filtered && !on_device)
+    if (filtered && !write_there)
         FTB_CHECK(cudaMemcpy2DAsync(filtered, io_row, d_filt, sizeof(float) * pitch, sizeof(float) * w,
                                     static_cast<size_t>(h) * n, out_kind, c.stream()));
     if (static_sky)
