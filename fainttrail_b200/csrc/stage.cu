@@ -940,8 +940,8 @@ __global__ void __launch_bounds__(N <= 64 ? 128 : 64) scatter_net_kernel(const S
     int c = 0;
 #pragma unroll
     for (int i = 0; i < N; ++i) c += finitef(v[i]);
-    if (c < a.n / 2) {
-        a.scatter[pix] = 1e9f;
+    if (c < a.n / 2 || c == 0) {  // (the median of no values is 0, with one frame)
+        a.scatter[pix] = c < a.n / 2 ? 1e9f : 0.0f;
         return;
     }
     uint32_t sv[N];
