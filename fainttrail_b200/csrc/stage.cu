@@ -32,6 +32,8 @@ namespace ftb {
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr double kFwhmToSigma = 1.0 / 2.354820045030949;  // psf.hpp:16
 
 __device__ __forceinline__ bool finitef(float v) { return isfinite(v); }
@@ -216,14 +218,18 @@ __global__ void __launch_bounds__(64) sky_kernel(const SkyArgs a) {
 // that enters takes the first free position from its run's first on, one that leaves
 // frees the run's first taken one; where a run reaches beyond the middle, its
 // count says which part the next one belongs to. Only the two zeros are equal and
-// differ: where the pixel holds a -0.0 and a median's value is zero, the wanted one is
-// looked up in rank order.
+// differ, which shows in the sky alone (a residual against one or the other differs at
+// most in the sign of a zero, which no sum, product or comparison after it sees): where
+// the pixel holds a -0.0 and its median is zero, the wanted one is looked up in rank
+// order.
 //
 // Bound by issue, mostly of the integer and compare pipe: 173 instructions a value at
 // 40 frames (a third of them in the loop over the ranks) where counting every rank
 // against all others and finishing on full masks took 330. 40 frames of 2048^2: 1.71
-// -> 1.02 ms; 120 of 1030 x 777 (a bitonic network, 64 threads a CTA with all
-// positions in shared memory): 5.46 -> 1.45 ms; 33 of 1501 x 1117: 0.57 -> 0.35 ms.
+// -> 1.01 ms; 120 of 1030 x 777 (a bitonic network, 64 threads a CTA with all
+// positions in shared memory): 5.46 -> 1.35 ms; 33 of 1501 x 1117: 0.57 -> 0.35 ms.
+// Whole numbers with a standard deviation of 33, most of whose pixels have equal values at
+// the middle's ends: 1.71 -> 1.45 and 7.59 -> 2.78 ms.
 
 // Masks: position of the lowest set bit (x != 0), of the k-th (0-based) set bit (k <
 // popc(x), x below 2^16 where small), and bit c, or 0 for a c beyond the mask.
@@ -367,27 +373,21 @@ __global__ void __launch_bounds__(sky_threads(N)) sky_middle_kernel(const SkyArg
             if (p >= first && p < first + len) to[p * T] = sv[p];
         for (int p = len; p < rows; ++p) S[p * T] = CUDART_INF_F;
     }
-    // the k-th value (0-based) in (value, time rank) order outside the window of rank r
-    // (r < -e: no window), which is a zero
-    auto zero = [&](int k, int r) {
-        for (int i = 0; i < n; ++i)
-            if (abs(i - r) > e) k -= value(i) < 0.0f;
-        float z = 0.0f;
+    // the k-th value (0-based) in (value, time rank) order; a zero is looked up, as its sign
+    // depends on the order
+    auto sorted = [&](int k) {
+        float z = S[(k - first) * T];
+        if (!negzero || z != 0.0f) return z;
+        for (int i = 0; i < n; ++i) k -= value(i) < 0.0f;
         for (int i = 0; i < n && k >= 0; ++i)
-            if (abs(i - r) > e && value(i) == 0.0f) {
+            if (value(i) == 0.0f) {
                 z = value(i);
                 --k;
             }
         return z;
     };
-    auto middle = [&](int pos, int k, int r) {
-        const float v = S[pos * T];
-        return negzero && v == 0.0f ? zero(k, r) : v;
-    };
     // global median: the two middle floats are added in float (preprocess.cpp:171)
-    const int far = -2 * n - e;
-    const double global = 0.5 * static_cast<double>(__fadd_rn(middle((m_all - 1) / 2 - first, (m_all - 1) / 2, far),
-                                                              middle(m_all / 2 - first, m_all / 2, far)));
+    const double global = 0.5 * static_cast<double>(__fadd_rn(sorted((m_all - 1) / 2), sorted(m_all / 2)));
     a.sky[pix] = __double2float_rn(global);
     if (e <= 0) {
         for (int r = 0; r < n; ++r) {
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(sky_threads(N)) sky_middle_kernel(const SkyArg
         out ^= up & (~up + 1);
     };
     for (int r = 0; r < e; ++r) enter(r < n ? code[r * T] : kNone, runs);
-    auto finish = [&](auto kind) {  // plain: no runs beyond the middle, no -0.0, five values kept always
+    auto finish = [&](auto kind) {  // plain: no runs beyond the middle, five values kept always
         constexpr bool kPlain = decltype(kind)::value;
         int m = m_all;
         if (!kPlain)
@@ -487,18 +487,14 @@ __global__ void __launch_bounds__(sky_threads(N)) sky_middle_kernel(const SkyArg
                 const int plo = nth_bit(kept, (u - 1) >> 1, rows <= 15);
                 const Mask above = kept & ~((static_cast<Mask>(2) << plo) - 1);
                 const int phi = u & 1 ? plo : low_bit(above);
-                float s0 = S[plo * T], s1 = S[phi * T];
-                if (!kPlain && negzero) {
-                    s0 = middle(plo, (m - 1) >> 1, r);
-                    s1 = middle(phi, m >> 1, r);
-                }
                 // double add of the two middle values (preprocess.cpp:198)
-                st = 0.5 * (static_cast<double>(s0) + static_cast<double>(s1));
+                st = 0.5 * (static_cast<double>(S[plo * T]) + static_cast<double>(S[phi * T]));
             }
             residual[at[r]] = v != CUDART_INF_F ? __double2float_rn(static_cast<double>(v) - st) : CUDART_NAN_F;
         }
     };
-    if (runs || negzero || a.need - X < 5)
+    // (the warp takes one of the two)
+    if (cg::coalesced_threads().any(runs || a.need - X < 5))
         finish(std::false_type());
     else
         finish(std::true_type());
@@ -600,7 +596,6 @@ __device__ __forceinline__ float key_value(uint32_t k) {
 // shared atomics on one of a few exponents' counters, measured 2.9 ms for 120 frames
 // of 790,000 samples; sampling and this 4.8 ms then, 0.75 ms now.
 
-namespace cg = cooperative_groups;
 constexpr int kSelCluster = 8;
 constexpr int kSelThreads = 512;
 constexpr int kSelList = 16384;  // keys a CTA keeps
