@@ -29,19 +29,6 @@ StreamPlan make_stream_plan(int w, int h, int n, const int* dx, const int* dy, i
     // clamped shifts: beyond +-w / +-h a frame never covers, as within
     auto X = [&](int j, size_t i) { return std::clamp(dx[static_cast<size_t>(j) * N + i], -w, w); };
     auto Y = [&](int j, size_t i) { return std::clamp(dy[static_cast<size_t>(j) * N + i], -h, h); };
-    // the frame whose shifts spread most orders the blocks
-    std::vector<int> lo(N, INT_MAX), hi(N, INT_MIN);
-    for (int j = 0; j < m; ++j) {
-        const int* a = dx + static_cast<size_t>(j) * N;
-        const int* b = dy + static_cast<size_t>(j) * N;
-        for (size_t i = 0; i < N; ++i) {
-            lo[i] = std::min(lo[i], std::min(a[i], b[i]));
-            hi[i] = std::max(hi[i], std::max(a[i], b[i]));
-        }
-    }
-    size_t ie = 0;
-    for (size_t i = 1; i < N; ++i)
-        if (static_cast<long long>(hi[i]) - lo[i] > static_cast<long long>(hi[ie]) - lo[ie]) ie = i;
     // classes of motions whose columns agree in every frame, each in index order
     std::vector<int> rep, chain;
     std::vector<std::vector<int>> members;
@@ -68,12 +55,16 @@ StreamPlan make_stream_plan(int w, int h, int n, const int* dx, const int* dy, i
     // most one step, of one row
     std::vector<Block> blocks;
     std::vector<int> stepped(N);
+    // pads cost what motions cost: up to a tenth of the slots
+    auto padded = [&]() {
+        const long long slots = static_cast<long long>(blocks.size()) * kStreamBlock;
+        return (slots - m) * 10 > slots;
+    };
     for (const std::vector<int>& mem : members) {
+        if (padded()) return P;  // (blocks only become more)
         Block b;
         auto close = [&]() {
             if (b.count == 0) return;
-            b.ex = X(b.motion[0], ie);
-            b.ey = Y(b.motion[0], ie);
             blocks.push_back(b);
             b.count = 0;
         };
@@ -94,9 +85,24 @@ StreamPlan make_stream_plan(int w, int h, int n, const int* dx, const int* dy, i
         }
         close();
     }
-    // pads cost what motions cost: up to a tenth of the slots
-    if ((static_cast<long long>(blocks.size()) * kStreamBlock - m) * 10 > static_cast<long long>(blocks.size()) * kStreamBlock)
-        return P;
+    if (padded()) return P;
+    // the frame whose shifts spread most orders the blocks
+    std::vector<int> lo(N, INT_MAX), hi(N, INT_MIN);
+    for (int j = 0; j < m; ++j) {
+        const int* a = dx + static_cast<size_t>(j) * N;
+        const int* b = dy + static_cast<size_t>(j) * N;
+        for (size_t i = 0; i < N; ++i) {
+            lo[i] = std::min(lo[i], std::min(a[i], b[i]));
+            hi[i] = std::max(hi[i], std::max(a[i], b[i]));
+        }
+    }
+    size_t ie = 0;
+    for (size_t i = 1; i < N; ++i)
+        if (static_cast<long long>(hi[i]) - lo[i] > static_cast<long long>(hi[ie]) - lo[ie]) ie = i;
+    for (Block& b : blocks) {
+        b.ex = X(b.motion[0], ie);
+        b.ey = Y(b.motion[0], ie);
+    }
     // groups of kStreamWarps blocks with close shifts: strips of columns about two
     // pixels wide at frame ie, each walked up or down in turn
     auto kx = [&](const Block& b) { return b.ex >> 1; };
