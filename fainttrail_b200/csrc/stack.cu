@@ -694,7 +694,7 @@ void StackPlanDev::upload(const StackPlan& p, cudaStream_t s) {
     unsigned char* base = static_cast<unsigned char*>(block);
     for (const Table& t : tables) *t.dst = base + t.at;
     // small tables by one copy; large ones from where they are (gathered first, the tables
-    // of 9008 motions and 100 frames took 5.6 ms to bring, now 0.45; the 60 KB of 212
+    // of 9008 motions and 100 frames took 5.6 ms to bring, now 0.45; the 20 KB of 212
     // motions and 16 frames 54 us either way)
     if (total <= kGatherBytes) {
         std::vector<unsigned char> host(total);

@@ -84,13 +84,16 @@ StreamPlan make_stream_plan(int w, int h, int n, const int* dx, const int* dy, i
     // most one step, of one row
     std::vector<Block> blocks;
     std::vector<int> stepped(N);
-    // pads cost what motions cost: up to a tenth of the slots
+    // pads cost what motions cost: up to a tenth of the slots, looked at before each class as
+    // if the motions left filled their blocks (slots only become more)
+    size_t left = static_cast<size_t>(m);
     auto padded = [&]() {
-        const long long slots = static_cast<long long>(blocks.size()) * kStreamBlock;
+        const long long slots = static_cast<long long>(blocks.size()) * kStreamBlock + static_cast<long long>(left);
         return (slots - m) * 10 > slots;
     };
     for (const std::vector<int>& mem : members) {
-        if (padded()) return P;  // (blocks only become more)
+        if (padded()) return P;
+        left -= mem.size();
         Block b;
         auto close = [&]() {
             if (b.count == 0) return;
