@@ -113,7 +113,8 @@ StackConfig choose_stack_config(int n, const int* dx, const int* dy, const std::
 
 // The streamed plan of a pass where `shape` asks for one (kStreamShape, or 0 and
 // the rule on its sizes) and its motions pack for it: `plan` and true, else false.
-// ahead: the plan is made while other passes run.
+// ahead: one of a batch's plans, made on host threads beside the others and mostly
+// while the device works.
 bool make_streamed_pass(int w, int h, int n, const int* dx, const int* dy, int m, int min_count, int shape, bool ahead,
                         StackPlan& plan);
 

@@ -2,12 +2,15 @@
 // build_stage (preprocess.cpp:286-486) for a whole image with a fixed PSF width,
 // bit-identical to the reference CPU code.
 //
-//  sky_kernel      static sky + leave-out residuals (preprocess.cpp:154-204)
+//  sky_middle_kernel, sky_kernel (more than 128 frames)
+//                  static sky + leave-out residuals (preprocess.cpp:154-204)
 //  sample + select per-frame residual noise: regular sample grid, exact medians
 //                  by bracketing and radix selection (common.hpp:64-100, preprocess.cpp:356-365)
-//  scatter_kernel  temporal scatter (preprocess.cpp:373-391)
+//  scatter_net_kernel, scatter_kernel (more than 128 frames)
+//                  temporal scatter (preprocess.cpp:373-391)
 //  mask_kernel     dilated scatter mask (preprocess.cpp:392-400)
-//  filter_kernel   normalise + weight, cosmic-ray rejection, clip, separable
+//  filter_frames_kernel, filter_kernel (wide PSFs)
+//                  normalise + weight, cosmic-ray rejection, clip, separable
 //                  matched filter, fused per tile (preprocess.cpp:414-451, 116-148)
 //  sample + select robust sigma of the filter output, then rescale
 //                  (preprocess.cpp:454-471)
@@ -44,8 +47,7 @@ struct SkyArgs {
     const float* sub;
     float* residual;
     float* sky;
-    const unsigned char* rank;         // time rank of each frame
-    const unsigned char* frame_of;     // frame of each time rank
+    const unsigned char* frame_of;  // frame of each time rank
     int w, h, pitch, n, exclude, need;
     int sub_pitch;  // of sub, any
 };
@@ -56,16 +58,16 @@ struct SkyArgs {
 // values per pass over the column (the non-finite ones are held as +inf and
 // never counted). The leave-out median of the frame of rank r is then the lo-th /
 // hi-th sorted value outside the exclusion window [r - exclude, r + exclude]; the
-// window's sorted positions are a bitmask of W words that slides one rank per
+// window's sorted positions are a bitmask that slides one rank per
 // frame (one position leaves, one enters), and the kept positions are picked
 // with popc / fns.
 // flips sorted position p (255: a non-finite value, no position) in the window
 // mask; returns 1 if a position was flipped
-template <int W>
-__device__ __forceinline__ int sky_toggle(uint32_t (&ex)[W], int p) {
+constexpr int kSkyWords = 8;  // 256 sorted positions
+__device__ __forceinline__ int sky_toggle(uint32_t (&ex)[kSkyWords], int p) {
     if (p == 255) return 0;
 #pragma unroll
-    for (int wd = 0; wd < W; ++wd) ex[wd] ^= (p >> 5) == wd ? 1u << (p & 31) : 0u;
+    for (int wd = 0; wd < kSkyWords; ++wd) ex[wd] ^= (p >> 5) == wd ? 1u << (p & 31) : 0u;
     return 1;
 }
 
@@ -88,7 +90,6 @@ __device__ __forceinline__ int nth_set_bit(uint32_t x, int k) {
 // The static sky and the leave-out residuals of one pixel from its values by
 // time rank (V, +inf where not finite), its m_all finite values in sorted order
 // (S) and each rank's sorted position (PF, 255 where not finite).
-template <int W>
 __device__ __forceinline__ void sky_finish(const SkyArgs& a, const float* V, const float* S, const unsigned char* PF,
                                            int T, int t, int m_all, size_t pix, size_t plane) {
     const int n = a.n;
@@ -96,16 +97,16 @@ __device__ __forceinline__ void sky_finish(const SkyArgs& a, const float* V, con
     const float mid_sum = __fadd_rn(S[((m_all - 1) / 2) * T + t], S[(m_all / 2) * T + t]);
     const double global = 0.5 * static_cast<double>(mid_sum);
     a.sky[pix] = __double2float_rn(global);
-    uint32_t ex[W];
+    uint32_t ex[kSkyWords];
 #pragma unroll
-    for (int wd = 0; wd < W; ++wd) ex[wd] = 0;
+    for (int wd = 0; wd < kSkyWords; ++wd) ex[wd] = 0;
     int excluded = 0;
     if (a.exclude > 0)
-        for (int r = 0; r <= min(a.exclude, n - 1); ++r) excluded += sky_toggle<W>(ex, PF[r * T + t]);  // rank 0's window
+        for (int r = 0; r <= min(a.exclude, n - 1); ++r) excluded += sky_toggle(ex, PF[r * T + t]);  // rank 0's window
     for (int r = 0; r < n; ++r) {
         if (a.exclude > 0 && r > 0) {
-            if (r - 1 - a.exclude >= 0) excluded -= sky_toggle<W>(ex, PF[(r - 1 - a.exclude) * T + t]);
-            if (r + a.exclude < n) excluded += sky_toggle<W>(ex, PF[(r + a.exclude) * T + t]);
+            if (r - 1 - a.exclude >= 0) excluded -= sky_toggle(ex, PF[(r - 1 - a.exclude) * T + t]);
+            if (r + a.exclude < n) excluded += sky_toggle(ex, PF[(r + a.exclude) * T + t]);
         }
         const float v = V[r * T + t];
         float* out = a.residual + a.frame_of[r] * plane + pix;
@@ -119,7 +120,7 @@ __device__ __forceinline__ void sky_finish(const SkyArgs& a, const float* V, con
             const int lo = (m - 1) / 2, hi = m / 2;
             int plo = -1, phi = -1, seen = 0;
 #pragma unroll
-            for (int wd = 0; wd < W; ++wd) {
+            for (int wd = 0; wd < kSkyWords; ++wd) {
                 const int nb = min(32, max(0, m_all - wd * 32));
                 const uint32_t valid = nb >= 32 ? 0xffffffffu : ((1u << nb) - 1u);
                 const uint32_t keep = ~ex[wd] & valid;
@@ -135,7 +136,6 @@ __device__ __forceinline__ void sky_finish(const SkyArgs& a, const float* V, con
     }
 }
 
-template <int W>
 __global__ void __launch_bounds__(64) sky_kernel(const SkyArgs a) {
     extern __shared__ unsigned char sm[];
     const int T = blockDim.x, t = threadIdx.x;
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(64) sky_kernel(const SkyArgs a) {
             PF[(e0 + b) * T + t] = fin ? static_cast<unsigned char>(pos[b]) : 255;
         }
     }
-    sky_finish<W>(a, V, S, PF, T, t, m_all, pix, plane);
+    sky_finish(a, V, S, PF, T, t, m_all, pix, plane);
 }
 
 // ---- the same for n <= N <= 128, without sorted positions for all values
@@ -890,7 +890,8 @@ __global__ void __launch_bounds__(128) scatter_kernel(const ScatterArgs a) {
 }
 
 // a / b to nearest from r = 1 / b to nearest, for finite a >= 0 and b > 0 of a size
-// that keeps quotient and remainders normal (a: a float, b: 1.4826 times one, or 1):
+// that keeps quotient and remainders normal (a: a float, b: 1.4826 times one, or 1; the
+// middle one of the deviations from a median does not exceed the largest float):
 // the quotient by r is corrected once to within a unit in the last place, and by
 // Markstein's theorem a second correction by its exact remainder rounds it correctly
 // (P. W. Markstein, IBM J. Res. Develop. 34, 1990). Five operations for the general
@@ -1002,27 +1003,16 @@ struct FilterArgs {
 // columns and the vertical pass. Pixels outside the image hold 0: a product with
 // 0 adds +0.0f to a sum that starts at +0.0f, which equals the reference's
 // truncated sums at the borders (preprocess.cpp:133-135, 140-145).
-// RT > 0: the filter radius fixed at compile time (the tile loops' index
-// arithmetic by constants, the taps in registers); RT = 0: any radius (a.R).
-// TWc x THc: the output tile.
-template <int RT, int TWc, int THc>
+// Any radius: the filter of wide PSFs (filter_frames_kernel has the others).
 __global__ void __launch_bounds__(256) filter_kernel(const FilterArgs a) {
     extern __shared__ float fs[];
-    const int R = RT > 0 ? RT : a.R, H = R + 2;
+    constexpr int TWc = 32, THc = 16;
+    const int R = a.R, H = R + 2;
     const int ZW = TWc + 2 * H, ZH = THc + 2 * H;
     float* Z = fs;                                    // ZH x ZW  z, then cleaned z
     unsigned char* F = reinterpret_cast<unsigned char*>(Z + ZW * ZH);  // ZH x ZW cosmic-ray centre flags
     float* Tt = reinterpret_cast<float*>(F + ((ZW * ZH + 15) / 16) * 16);  // (THc + 2R) x TWc horizontal pass
     __shared__ int cr_tile;
-    constexpr int KN = RT > 0 ? 2 * RT + 1 : 1;
-    float kr[KN], kn[KN];  // taps and taps x norm (the reference's float product) when RT > 0
-    if constexpr (RT > 0) {
-#pragma unroll
-        for (int j = 0; j < KN; ++j) {
-            kr[j] = a.k[j];
-            kn[j] = __fmul_rn(kr[j], a.norm);
-        }
-    }
     const int f = blockIdx.z;
     const int x0 = blockIdx.x * TWc, y0 = blockIdx.y * THc;
     const size_t plane = static_cast<size_t>(a.pitch) * a.h;
@@ -1091,12 +1081,7 @@ __global__ void __launch_bounds__(256) filter_kernel(const FilterArgs a) {
         const int c = e % TWc, r = e / TWc;
         const float* row = Zc + (r + 2) * ZW + (c + 2);  // centre column at H + c, row at 2 + r (= H - R + r)
         float acc = 0.0f;
-        if constexpr (RT > 0) {
-#pragma unroll
-            for (int j = 0; j < KN; ++j) acc = __fadd_rn(acc, __fmul_rn(row[j], kr[j]));
-        } else {
-            for (int j = 0; j <= 2 * R; ++j) acc = __fadd_rn(acc, __fmul_rn(row[j], a.k[j]));
-        }
+        for (int j = 0; j <= 2 * R; ++j) acc = __fadd_rn(acc, __fmul_rn(row[j], a.k[j]));
         const int gy = y0 - R + r;
         Tt[e] = (gy >= 0 && gy < a.h) ? acc : 0.0f;
     }
@@ -1106,22 +1091,15 @@ __global__ void __launch_bounds__(256) filter_kernel(const FilterArgs a) {
         const int gx = x0 + c, gy = y0 + r;
         if (gx >= a.w || gy >= a.h) continue;
         float acc = 0.0f;
-        if constexpr (RT > 0) {
-#pragma unroll
-            for (int j = 0; j < KN; ++j) acc = __fadd_rn(acc, __fmul_rn(kn[j], Tt[(r + j) * TWc + c]));
-        } else {
-            for (int j = 0; j <= 2 * R; ++j)
-                acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(a.k[j], a.norm), Tt[(r + j) * TWc + c]));
-        }
+        // (the taps times the norm: the reference's float product)
+        for (int j = 0; j <= 2 * R; ++j)
+            acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(a.k[j], a.norm), Tt[(r + j) * TWc + c]));
         a.out[f * plane + static_cast<size_t>(gy) * a.pitch + gx] = acc;
     }
     __syncthreads();
     if (threadIdx.x == 0 && cr_tile) atomicAdd(&a.cr[f], cr_tile);
 }
 
-// the static sky: counted ranks up to 64 frames (measured faster there: 554
-// against 375 GB/s at 40 frames), the sorting network up to 128 (where the
-// counting grows with n^2), counted ranks beyond
 template <int N, class Mask>
 void launch_sky_middle(const SkyArgs& a, long long npix, cudaStream_t s) {
     constexpr int T = sky_threads(N);
@@ -1143,8 +1121,8 @@ void launch_sky(const SkyArgs& a, int n, long long npix, cudaStream_t s) {
     if (n > 128 || npix > 0x7fffffffLL) {
         const int T = 64;
         const size_t smem = static_cast<size_t>(T) * n * 9;
-        allow_dynamic_smem(reinterpret_cast<const void*>(sky_kernel<8>), smem);
-        sky_kernel<8><<<static_cast<unsigned>((npix + T - 1) / T), T, smem, s>>>(a);
+        allow_dynamic_smem(reinterpret_cast<const void*>(sky_kernel), smem);
+        sky_kernel<<<static_cast<unsigned>((npix + T - 1) / T), T, smem, s>>>(a);
         FTB_CHECK(cudaGetLastError());
     } else if (middle > 64) {
         launch_sky_middle<128, unsigned __int128>(a, npix, s);
@@ -1440,14 +1418,12 @@ void launch_filter_frames(const FilterArgs& a, int n, int sms, cudaStream_t s) {
     FTB_CHECK(cudaGetLastError());
 }
 
-// one launch of the filter kernel for radius R (compile-time radius up to 8)
-template <int RT, int TWc, int THc>
 void launch_filter(const FilterArgs& a, int n, cudaStream_t s) {
-    const int R = RT > 0 ? RT : a.R, H = R + 2, ZW = TWc + 2 * H, ZH = THc + 2 * H;
+    constexpr int TWc = 32, THc = 16;
+    const int R = a.R, H = R + 2, ZW = TWc + 2 * H, ZH = THc + 2 * H;
     const size_t smem = sizeof(float) * ZW * ZH + ((ZW * ZH + 15) / 16) * 16 + sizeof(float) * (THc + 2 * R) * TWc;
-    auto kern = filter_kernel<RT, TWc, THc>;
-    allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
-    kern<<<dim3((a.w + TWc - 1) / TWc, (a.h + THc - 1) / THc, n), 256, smem, s>>>(a);
+    allow_dynamic_smem(reinterpret_cast<const void*>(filter_kernel), smem);
+    filter_kernel<<<dim3((a.w + TWc - 1) / TWc, (a.h + THc - 1) / THc, n), 256, smem, s>>>(a);
     FTB_CHECK(cudaGetLastError());
 }
 
@@ -1461,7 +1437,7 @@ void launch_filter_any(const FilterArgs& a, int n, int sms, cudaStream_t s) {
         case 6: launch_filter_frames<6>(a, n, sms, s); break;
         case 7: launch_filter_frames<7>(a, n, sms, s); break;
         case 8: launch_filter_frames<8>(a, n, sms, s); break;
-        default: launch_filter<0, 32, 16>(a, n, s); break;
+        default: launch_filter(a, n, s); break;
     }
 }
 
@@ -1618,9 +1594,6 @@ int sample_grid_points(int w, int h, int border) {
     return st > 0 ? grid_count(border, w - border, st) * grid_count(border, h - border, st) : 0;
 }
 
-namespace {
-}  // namespace
-
 int filter_border(double fwhm_px) { return static_cast<int>(std::ceil(3 * fwhm_px * kFwhmToSigma)) + 1; }
 
 StageScratch::StageScratch(Context& c, int w, int h, int n, double fwhm_px) : w_(w), h_(h), n_(n) {
@@ -1632,7 +1605,7 @@ StageScratch::StageScratch(Context& c, int w, int h, int n, double fwhm_px) : w_
     cap = std::max(1, sample_grid_points(w, h, filter_border(fwhm_px)));
     for (int b = 0; b <= 64; ++b) cap = std::max(cap, sample_grid_points(w, h, b));
     samples = DevBuf(&c, sizeof(float) * static_cast<size_t>(cap) * n, "noise samples");
-    small = DevBuf(&c, 4096 + sizeof(double) * 2 * n + sizeof(int) * 2 * n + 2 * static_cast<size_t>(n), "stage tables");
+    small = DevBuf(&c, 4096 + sizeof(double) * 2 * n + sizeof(int) * 2 * n + static_cast<size_t>(n), "stage tables");
 }
 
 bool StageScratch::fits(int w, int h, int n, double fwhm_px) const {
@@ -1642,14 +1615,14 @@ bool StageScratch::fits(int w, int h, int n, double fwhm_px) const {
 bool StageScratch::holds(int w, int h, int n) const { return w == w_ && h <= h_ && n == n_; }
 
 // The device tables of a stage in StageScratch::small: filter taps, per-frame
-// sigma, filter sigma, sample counts, cosmic-ray tallies, rank tables.
+// sigma, filter sigma, sample counts, cosmic-ray tallies, the frame of each time rank.
 struct StageTables {
     float* taps;
     double* sigma;
     double* sg;
     int* counts;
     int* cr;
-    unsigned char* tab;
+    unsigned char* frame_of;
 };
 
 static StageTables stage_tables(StageScratch& sc, int n) {
@@ -1660,7 +1633,7 @@ static StageTables stage_tables(StageScratch& sc, int n) {
     t.sg = t.sigma + n;
     t.counts = reinterpret_cast<int*>(t.sg + n);
     t.cr = t.counts + n;
-    t.tab = reinterpret_cast<unsigned char*>(t.cr + n);
+    t.frame_of = reinterpret_cast<unsigned char*>(t.cr + n);
     return t;
 }
 
@@ -1674,21 +1647,18 @@ void stage_noise(Context& c, StageScratch& sc, const float* d_sub, int w, int h,
     cudaStream_t s = c.stream();
     const StageTables tb = stage_tables(sc, n);
 
-    // host tables: time ranks and the frame of each rank
+    // the frame of each time rank
     std::vector<int> rank;
     stage_time_ranks(t_h, n, rank);
     const int exclude = static_exclude >= 0 ? static_exclude : std::max(1, static_cast<int>(std::lround(n / 8.0)));
-    std::vector<unsigned char> tab(2 * static_cast<size_t>(n));
-    for (int i = 0; i < n; ++i) {
-        tab[static_cast<size_t>(i)] = static_cast<unsigned char>(rank[static_cast<size_t>(i)]);
-        tab[static_cast<size_t>(n + rank[static_cast<size_t>(i)])] = static_cast<unsigned char>(i);
-    }
-    FTB_CHECK(cudaMemcpyAsync(tb.tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, s));
+    std::vector<unsigned char> frame_of(static_cast<size_t>(n));
+    for (int i = 0; i < n; ++i) frame_of[static_cast<size_t>(rank[static_cast<size_t>(i)])] = static_cast<unsigned char>(i);
+    FTB_CHECK(cudaMemcpyAsync(tb.frame_of, frame_of.data(), frame_of.size(), cudaMemcpyHostToDevice, s));
     FTB_CHECK(cudaMemsetAsync(tb.counts, 0, sizeof(int) * 2 * n, s));  // counts and cosmic-ray tallies
     // 1. static sky + residuals
     {
         const int span = c.span_begin("static sky + residuals");
-        SkyArgs a{d_sub, sc.residual.as<float>(), d_sky, tb.tab, tb.tab + n, w, h, pitch, n, exclude,
+        SkyArgs a{d_sub, sc.residual.as<float>(), d_sky, tb.frame_of, w, h, pitch, n, exclude,
                   std::max(5, static_cast<int>(0.6 * n)), sub_pitch > 0 ? sub_pitch : pitch};
         launch_sky(a, n, npix, s);
         ++c.launches;
@@ -1810,7 +1780,6 @@ void stage_sigma_to_host(Context& c, StageScratch& sc, int n, double* h_sigma) {
 void prepare_sub(Context& c, StageScratch& sc, const float* d_raw, float* d_sub, int w, int h, int n, double* h_bg) {
     const int pitch = frame_pitch(w);
     const size_t plane = static_cast<size_t>(pitch) * h;
-    const long long npix = static_cast<long long>(w) * h;
     cudaStream_t s = c.stream();
     const StageTables tb = stage_tables(sc, n);
     const int span = c.span_begin("background + borders");
@@ -1841,14 +1810,11 @@ void stage_sky(Context& c, StageScratch& sc, const float* d_sub, int w, int rows
     std::vector<int> rank;
     stage_time_ranks(t_h, n, rank);
     const int exclude = static_exclude >= 0 ? static_exclude : std::max(1, static_cast<int>(std::lround(n / 8.0)));
-    std::vector<unsigned char> tab(2 * static_cast<size_t>(n));
-    for (int i = 0; i < n; ++i) {
-        tab[static_cast<size_t>(i)] = static_cast<unsigned char>(rank[static_cast<size_t>(i)]);
-        tab[static_cast<size_t>(n + rank[static_cast<size_t>(i)])] = static_cast<unsigned char>(i);
-    }
-    FTB_CHECK(cudaMemcpyAsync(tb.tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, s));
+    std::vector<unsigned char> frame_of(static_cast<size_t>(n));
+    for (int i = 0; i < n; ++i) frame_of[static_cast<size_t>(rank[static_cast<size_t>(i)])] = static_cast<unsigned char>(i);
+    FTB_CHECK(cudaMemcpyAsync(tb.frame_of, frame_of.data(), frame_of.size(), cudaMemcpyHostToDevice, s));
     const int span = c.span_begin("static sky + residuals");
-    SkyArgs a{d_sub, sc.residual.as<float>(), d_sky, tb.tab, tb.tab + n, w, rows, pitch, n, exclude,
+    SkyArgs a{d_sub, sc.residual.as<float>(), d_sky, tb.frame_of, w, rows, pitch, n, exclude,
               std::max(5, static_cast<int>(0.6 * n)), pitch};
     launch_sky(a, n, npix, s);
     ++c.launches;
