@@ -388,6 +388,12 @@ def reference_arm(args):
     rank, _, world = env_rank()
     if rank != 0:
         return
+    sys.path.insert(0, os.path.join(ROOT, "tests"))
+    from ftoracle import REF_DRIVER_SO
+    if not os.path.exists(REF_DRIVER_SO):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference is not built here (make -C oracle ref)"}),
+              flush=True)
+        return
     from fainttrail_b200 import synthetic
     wl = synthetic.WORKLOADS[args.workload]
     import torch
