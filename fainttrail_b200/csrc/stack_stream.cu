@@ -10,17 +10,18 @@
 // group after group and tile after tile follow without a pause. A lane loads its
 // column of a frame's window once, 17 rows, and adds it to all five motions.
 //
-// What bounds it: issue. A paired add (add.rn.f32x2) holds the issue port for two
-// cycles, as two single adds do, so 128 adds a cycle and SM is reached only if
-// nothing else issues; loads, descriptors and branches take an add's place. Five
-// motions a load and not four: 40 paired adds beside about 45 other instructions
-// (micro-measured, loads, descriptor, branches and loop) where four motions have 32
-// beside 60. More motions need more than the 128 registers that sixteen warps
-// have; fewer warps leave the load latency open (blocks of eight on eight warps
-// 9 T adds/s). Measured: 15.4 T adds/s at 120 frames of 2048 x 1024 (462 ms; 32 x 8
-// and 32 x 4 tiles with resident windows 1080), 14.3 T at 40 frames of 2048^2 (46.4
-// ms; resident windows 42.4), 40 paired adds a block and frame beside 70 other issue
-// slots, 5 % of the time in the maxima and 7 % waiting for copies.
+// What bounds it: issue and the FMA pipe, with four warps a scheduler. A paired add
+// (add.rn.f32x2) takes the pipe for two cycles, as two single adds do, so 128 adds a
+// cycle and SM need every other cycle's issue slot and leave the rest to loads,
+// descriptors and branches. A block and frame takes 105 instructions with its share of
+// the maxima, 40 of them the adds (120 frames of 1024 x 512: issue active 57 % of the
+// cycles, the FMA pipe 50 %; stalls on fixed latencies 2.0 an issue, on loads and the
+// copies 1.5, on the pipe 0.7). Five motions a load and not four, which have 32 adds
+// beside the same loads; more need more than the 128 registers that sixteen warps have;
+// fewer warps leave the load latency open (blocks of eight on eight warps 9 T adds/s).
+// Measured: 15.4 T adds/s at 120 frames of 2048 x 1024 (462 ms; 32 x 8 and 32 x 4 tiles
+// with resident windows 1080), 14.3 T at 40 frames of 2048^2 (46.4 ms; resident windows
+// 42.4).
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
