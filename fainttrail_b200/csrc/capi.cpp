@@ -252,7 +252,7 @@ namespace {
 // choice; passes planned with others stream up to another size, make_streamed_pass);
 // a shape that does not take the pass falls back to the automatic choice, as
 // ft_b200_set_tile_shape does for the device.
-ftb::StackPlan plan_on_host(int w, int h, int n, const int* dx, const int* dy, int m, int min_count, int shape) {
+static ftb::StackPlan plan_on_host(int w, int h, int n, const int* dx, const int* dy, int m, int min_count, int shape) {
     constexpr int kB200SmemOptin = 232448;  // 227 KB of shared memory per block
     ftb::StackPlan plan;
     if (ftb::make_streamed_pass(w, h, n, dx, dy, m, min_count, shape, false, plan)) return plan;
